@@ -195,20 +195,59 @@ __device__ __forceinline__ double div_r(double a, double b) { return __ddiv_rn(a
 __device__ __forceinline__ float rcp_r(float x) { return __frcp_rn(x); }
 __device__ __forceinline__ double rcp_r(double x) { return __drcp_rn(x); }
 
+// a > b ? a : b
+__device__ __forceinline__ float above_r(float a, float b) { return a > b ? a : b; }
+__device__ __forceinline__ double above_r(double a, double b) { return a > b ? a : b; }
+
+// Two cells' FP32 values as one arithmetic type.  sm_100 has two-wide FP32
+// multiplies, adds and fused multiply-adds (each half one IEEE operation,
+// rounded like the scalar one), so a thread that owns two cells issues half
+// the arithmetic instructions and every result keeps its bits.  The 16-bit
+// steps are bound by instruction issue, not by HBM: this is what they need.
+template <class R>
+struct Scalar {
+  using T = R;
+};
+struct F2 {
+  float2 v;
+  F2() = default;
+  __device__ __forceinline__ F2(float lo, float hi) : v(make_float2(lo, hi)) {}
+  __device__ __forceinline__ F2(float x) : v(make_float2(x, x)) {}
+  __device__ __forceinline__ F2(double x) : F2(static_cast<float>(x)) {}
+  __device__ __forceinline__ F2(int x) : F2(static_cast<float>(x)) {}
+  __device__ __forceinline__ F2 operator-() const { return F2(-v.x, -v.y); }
+};
+template <>
+struct Scalar<F2> {
+  using T = float;
+};
+__device__ __forceinline__ F2 f2(float2 v) { return F2(v.x, v.y); }
+__device__ __forceinline__ F2 fma_r(F2 a, F2 b, F2 c) { return f2(__ffma2_rn(a.v, b.v, c.v)); }
+__device__ __forceinline__ F2 mul_r(F2 a, F2 b) { return f2(__fmul2_rn(a.v, b.v)); }
+__device__ __forceinline__ F2 add_r(F2 a, F2 b) { return f2(__fadd2_rn(a.v, b.v)); }
+// a - b as (-1) b + a: one two-wide instruction, rounded once, the same value
+__device__ __forceinline__ F2 sub_r(F2 a, F2 b) { return fma_r(b, F2(-1.0f), a); }
+__device__ __forceinline__ F2 rcp_r(F2 a) { return F2(rcp_r(a.v.x), rcp_r(a.v.y)); }
+__device__ __forceinline__ F2 above_r(F2 a, F2 b) {
+  return F2(above_r(a.v.x, b.v.x), above_r(a.v.y, b.v.y));
+}
+
 // sum_a s_a x_a over the nonzero components s_a = +-1 of a direction (exact
-// sign flips; the additions are rounded in axis order).
+// sign flips; the additions are rounded in axis order; -a + b is taken as
+// b - a, the same value without a sign flip of its own).
 template <class R>
 __device__ __forceinline__ R dot_e(int e0, int e1, int e2, const R (&x)[3]) {
-  R v = 0;
-  bool first = true;
   const int e[3] = {e0, e1, e2};
+  int i[3] = {0, 0, 0}, n = 0;
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    if (e[k] == 0) continue;
-    const R t = e[k] > 0 ? x[k] : -x[k];
-    v = first ? t : add_r(v, t);
-    first = false;
-  }
+  for (int k = 0; k < 3; ++k)
+    if (e[k] != 0) i[n++] = k;
+  if (n == 0) return R(0);
+  if (n == 1) return e[i[0]] > 0 ? x[i[0]] : -x[i[0]];
+  R v;
+  if (e[i[0]] > 0) v = e[i[1]] > 0 ? add_r(x[i[0]], x[i[1]]) : sub_r(x[i[0]], x[i[1]]);
+  else v = e[i[1]] > 0 ? sub_r(x[i[1]], x[i[0]]) : sub_r(-x[i[0]], x[i[1]]);
+  if (n == 3) v = e[i[2]] > 0 ? add_r(v, x[i[2]]) : sub_r(v, x[i[2]]);
   return v;
 }
 
@@ -311,13 +350,17 @@ __device__ __forceinline__ Mom<R> moments(const R (&d)[Q], const R (&F)[3], bool
     const R w = static_cast<R>(Lat<Q>::wr(q));
     const R s = add_r(d[q], d[o]);
     const R t = sub_r(d[q], d[o]);
-    rdp = fma_r(w, s, rdp);
+    rdp = Lat<Q>::wr(q) == 1 ? add_r(rdp, s) : fma_r(w, s, rdp);
     const int e[3] = {Lat<Q>::c0(q), Lat<Q>::c1(q), Lat<Q>::c2(q)};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       if (e[k] == 0) continue;
-      const R ws = e[k] > 0 ? w : -w;
-      m[k] = used[k] ? fma_r(ws, t, m[k]) : mul_r(ws, t);
+      if (used[k] && Lat<Q>::wr(q) == 1) {  // +-1 t: one rounded addition
+        m[k] = e[k] > 0 ? add_r(m[k], t) : sub_r(m[k], t);
+      } else {
+        const R ws = static_cast<R>(e[k] > 0 ? Lat<Q>::wr(q) : -Lat<Q>::wr(q));
+        m[k] = used[k] ? fma_r(ws, t, m[k]) : mul_r(ws, t);
+      }
       used[k] = true;
     }
   }
@@ -328,12 +371,13 @@ __device__ __forceinline__ Mom<R> moments(const R (&d)[Q], const R (&F)[3], bool
     }
   }
   // 1/36 = c_hi + c_lo to twice the working precision
-  constexpr R c_hi = static_cast<R>(1.0 / kDen);
-  constexpr R c_lo = static_cast<R>(1.0 / kDen - static_cast<double>(c_hi));
+  using S = typename Scalar<R>::T;
+  constexpr S c_hi = static_cast<S>(1.0 / kDen);
+  constexpr S c_lo = static_cast<S>(1.0 / kDen - static_cast<double>(c_hi));
   Mom<R> r;
-  r.rd = fma_r(rdp, c_hi, mul_r(rdp, c_lo));
+  r.rd = fma_r(rdp, R(c_hi), mul_r(rdp, R(c_lo)));
   r.rho = add_r(R(1), r.rd);
-  const R den = r.rho > R(1e-10) ? r.rho : R(1e-10);
+  const R den = above_r(r.rho, R(1e-10));
   const R inv = rcp_r(mul_r(static_cast<R>(kDen), den));  // 1 / (36 rho)
 #pragma unroll
   for (int k = 0; k < 3; ++k) r.u[k] = mul_r(m[k], inv);
@@ -360,13 +404,14 @@ __device__ __forceinline__ void collide(R (&d)[Q], const Mom<R>& m, const R (&F)
   const R r45 = mul_r(R(4.5), orho);
   const R r3 = mul_r(R(3), orho);
   const R keep = sub_r(R(1), omega);
-  R c3 = 0, c9 = 0, cuF = 0, even0 = base;
+  R c3 = 0, c9 = 0, ncuF = 0, even0 = base;
+  const R n3 = mul_r(R(-3), orho);
   if constexpr (FORCE) {
     const R uF = fma_r(m.u[0], F[0], fma_r(m.u[1], F[1], mul_r(m.u[2], F[2])));
     c3 = mul_r(R(3), guo_c);
     c9 = mul_r(R(9), guo_c);
-    cuF = mul_r(c3, uF);  // c 3 u.F
-    even0 = sub_r(base, cuF);
+    ncuF = mul_r(-c3, uF);  // -c 3 u.F
+    even0 = add_r(base, ncuF);
   }
   d[0] = fma_r(keep, d[0], even0);
 #pragma unroll
@@ -382,14 +427,14 @@ __device__ __forceinline__ void collide(R (&d)[Q], const Mom<R>& m, const R (&F)
       const R eF = dot_e(e0, e1, e2, F);
       const R c9eF = mul_r(c9, eF), c3eF = mul_r(c3, eF);
       R A = fma_r(r45, mul_r(eu, eu), base);
-      A = add_r(A, fma_r(eu, c9eF, -cuF));
+      A = add_r(A, fma_r(eu, c9eF, ncuF));
       const R B = fma_r(r3, eu, c3eF);
       d[q] = add_r(fma_r(keep, dq, A), B);
       d[o] = sub_r(fma_r(keep, dop, A), B);
     } else {
       // (1 - omega) d + base + eu (4.5 omega rho eu +- 3 omega rho)
       d[q] = fma_r(eu, fma_r(r45, eu, r3), fma_r(keep, dq, base));
-      d[o] = fma_r(eu, fma_r(r45, eu, -r3), fma_r(keep, dop, base));
+      d[o] = fma_r(eu, fma_r(r45, eu, n3), fma_r(keep, dop, base));
     }
   }
 }
@@ -678,8 +723,8 @@ __device__ __forceinline__ R to_offset(R f, int q) {
 }
 template <int Q, class R>
 __device__ __forceinline__ R from_offset(R d, int q) {
-  if constexpr (sizeof(R) == 8) return fma_r(Lat<Q>::w(q), d, Lat<Q>::w(q));
-  else return add_r(w_hi<Q>(q), fma_r(w_hi<Q>(q), d, w_lo<Q>(q)));
+  if constexpr (sizeof(typename Scalar<R>::T) == 8) return fma_r(Lat<Q>::w(q), d, Lat<Q>::w(q));
+  else return add_r(R(w_hi<Q>(q)), fma_r(R(w_hi<Q>(q)), d, R(w_lo<Q>(q))));
 }
 
 // Collide from a reference-layout state f (*grid_shape, Q): p = C(f).

@@ -44,31 +44,24 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
       : "memory");
 }
 
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// This CTA's shared memory -> global, `bytes` a multiple of 16, both addresses
-// 16-byte aligned; tracked in the issuing thread's bulk async-group, which
-// this call commits.
-__device__ __forceinline__ void bulk_store_s2g(void* dst, const void* src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
-               "r"(smem_u32(src)), "r"(bytes)
+// Two runs of this CTA's shared memory -> global (the second one may be empty),
+// sizes multiples of 16, addresses 16-byte aligned; tracked as one bulk
+// async-group of the issuing thread, which this call commits.
+__device__ __forceinline__ void bulk_store2_s2g(void* dst0, const void* src0, uint32_t bytes0,
+                                                void* dst1, const void* src1, uint32_t bytes1) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst0),
+               "r"(smem_u32(src0)), "r"(bytes0)
                : "memory");
+  if (bytes1 > 0)
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst1),
+                 "r"(smem_u32(src1)), "r"(bytes1)
+                 : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 
-// All but the issuing thread's most recent bulk store have finished reading
-// shared memory.
-__device__ __forceinline__ void bulk_wait_read_1() {
-  asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+// The issuing thread's bulk stores have finished reading shared memory.
+__device__ __forceinline__ void bulk_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
 // The issuing thread's bulk stores are complete.

@@ -13,20 +13,19 @@
 //   * Each plane of the column, with a one-cell halo on every side, is moved
 //     from the reference layout into a ring of shared-memory slots by the copy
 //     engine (1-D bulk asynchronous copies, cp.async.bulk, completion on an
-//     mbarrier).  A tile row is copied as whole groups of four cells (a
-//     16-byte multiple for Q x 4 B), kTileHalo = 4 cells on each side, with the
-//     periodic wrap as separate copies.
+//     mbarrier); the periodic wrap along a row is a copy of its own.
 //   * Warps have one role each and meet only at mbarriers, never at a block
 //     barrier: a producer warp issues the copies of plane P once the slot's
 //     previous plane is consumed; collide warps collide plane P in place
-//     (every tile and halo cell, k_prepare's arithmetic) once it has landed;
-//     output warps, one per 32-cell tile row, pull the collided populations of
-//     plane P from slots P - 1, P, P + 1 once P + 1 is collided, apply the
-//     wall swap and the faces, take the moments and write f_bc (kOutAoS:
-//     staged per warp in shared memory, two staging rows used in turn, and
-//     written by a bulk asynchronous store) or collide again and write the
-//     next state planes (kOutState: the first step of a rollout).  Collide warps run up
-//     to a few planes ahead of the output warps.
+//     (every tile and halo cell, k_prepare's arithmetic, two cells per lane
+//     with two-wide FP32 arithmetic) once it has landed and keep the wall
+//     bits of its cells beside it; output warps, each over 32 or 64 cells of
+//     the tile, pull the collided populations of plane P from slots P - 1, P,
+//     P + 1 once P + 1 is collided, apply the wall swap and the faces, take
+//     the moments and write f_bc (kOutAoS: staged per warp in shared memory
+//     and written by a bulk asynchronous store) or collide again and write
+//     the next state planes (kOutState: the first step of a rollout).
+//     Collide warps run up to a few planes ahead of the output warps.
 //   * A persistent grid walks work items (column, chunk of planes along the
 //     sweep); blocks take items with a grid stride in chunk-major order, so
 //     neighbouring columns are swept at the same time and the halo rows they
@@ -44,78 +43,102 @@
 // own copies in flight and returns.
 #pragma once
 
+#include <type_traits>
+
 #include "lbm_kernels.cuh"
+#include "lbm_pair.cuh"
 #include "lbm_staged.cuh"
 
 namespace lbm {
 
 // Tile shape, warp roles and sweep mapping per lattice.
+//
+// What bounds the kernel is the chain of dependent instructions in the collide
+// and output warps, at the few warps that one ring of planes leaves room for:
+// both are busy for 0.8-0.9 of the launch, which issues on 0.58 of the cycles
+// with DRAM at 0.43 (160^2 x 128).  One update, measured side by side:
+//   D3Q19, 256^3 with spheres and faces / channel with a force: 0.59 / 0.66 ms
+//   (0.68 / 0.68 before, with five slots of 37 KB -- whole groups of four halo
+//   cells -- and collide lanes that run one cell after the other).  The ring
+//   takes six planes of 10 + 2 rows at 31 KB: three read, one collided, two
+//   landing.  Two cells per output lane: 0.70 / 0.62 (half the warps); the same
+//   in two groups of warps on alternate planes of 8 rows: 0.65 / 0.69; 12 rows in
+//   five slots: 0.69 / 0.71; 13 collide warps of one cell per lane: 0.73 / 0.61
+//   (80 registers, spills).
+//   D2Q9, 4096^2: 0.276 ms (0.41 before): its planes are small, so three blocks
+//   of nine warps share an SM.  252 cells per row: the 254 collided cells fill
+//   four warps.  124 cells in six blocks: 0.293; 252 in two or four: 0.32, 0.31.
 template <int Q>
 struct Sweep;
 template <>
 struct Sweep<19> {
-  static constexpr int TY = 10, TZ = 32;  // tile rows (a1) x row cells (a2)
-  static constexpr int HR = 1;            // halo rows
-  static constexpr int NCW = 8;           // collide warps, two cells per lane over the
-  static constexpr int CPL = 2;           //   (10 + 2) x 40 buffered cells <= 8 x 32 x 2
-  static constexpr int MINB = 1;          // resident blocks per SM
-  // plane slots: 3 read by the output warps, one being collided, one landing
-  // (the ring and two staging rows per output warp fill 226 KB of shared memory)
-  static constexpr int SLOTS = 5;
+  static constexpr int TY = 10, TZ = 32;    // tile rows (a1) x row cells (a2)
+  static constexpr int HR = 1;              // halo rows
+  static constexpr int CPO = 1;             // cells per output lane
+  static constexpr int OZ = 0;              // its second cell: that many cells further
+  static constexpr int NOW = 10;            // output warps
+  static constexpr int SLOTS = 6;           // plane slots
+  static constexpr int MINB = 1;            // resident blocks per SM
   __host__ __device__ static constexpr int cs(int q) { return Lat<19>::c0(q); }  // sweep
   __host__ __device__ static constexpr int cr(int q) { return Lat<19>::c1(q); }  // rows
 };
 template <>
 struct Sweep<9> {
-  static constexpr int TY = 1, TZ = 128;
+  static constexpr int TY = 1, TZ = 252;
   static constexpr int HR = 0;
-  static constexpr int NCW = 3;  // 136 buffered cells <= 3 x 32 x 2
-  static constexpr int CPL = 2;
-  static constexpr int MINB = 2;
-  static constexpr int SLOTS = 6;  // two planes landing ahead of the collide
+  static constexpr int CPO = 2;
+  static constexpr int OZ = 128;
+  static constexpr int NOW = 4;
+  static constexpr int SLOTS = 6;
+  static constexpr int MINB = 3;
   __host__ __device__ static constexpr int cs(int q) { return Lat<9>::c1(q); }
   __host__ __device__ static constexpr int cr(int) { return 0; }
 };
 
-constexpr int kTileHalo = 4;   // cells copied on each side of a tile row
-constexpr int kMaxTileSlots = 6;  // plane slots of the deepest ring (Sweep<Q>::SLOTS)
-
 template <int Q>
 struct TileShape {
   static constexpr int TY = Sweep<Q>::TY, TZ = Sweep<Q>::TZ, HR = Sweep<Q>::HR;
-  static constexpr int W = TZ + 2 * kTileHalo;        // cells per buffered row
   static constexpr int RP = TY + 2 * HR;              // buffered rows per plane
-  static constexpr int CW = TZ + 2;                   // collided cells per row
-  static constexpr int PLANE = RP * W * Q;            // IO elements per plane slot
-  static constexpr int NCW = Sweep<Q>::NCW;           // collide warps
-  static constexpr int CPL = Sweep<Q>::CPL;           // cells per collide lane
-  static constexpr int NOW = TY * TZ / 32;            // output warps (32 cells each)
+  static constexpr int CW = TZ + 2;                   // buffered (= collided) cells per row
+  // A buffered row: the halo cell before the tile, the tile's cells, the halo
+  // cell after it, copied in whole 16-byte units.  Tile rows start on groups of
+  // four cells (4 Q x 4 B is a multiple of 16), so the cell before the tile ends
+  // on a 16-byte boundary and the cell after it starts on one.
+  static constexpr int LCH = (Q + 3) / 4 * 4;         // words of either halo cell's copy
+  static constexpr int RW = LCH + TZ * Q + LCH;       // words per buffered row
+  static constexpr int PLANE = RP * RW;               // words per plane slot
+  static constexpr int NCW = (RP * CW + 63) / 64;     // collide warps, two cells per lane
+  static constexpr int NOW = Sweep<Q>::NOW, CPO = Sweep<Q>::CPO, OZ = Sweep<Q>::OZ;
   static constexpr int NT = 32 * (1 + NCW + NOW);     // + the producer warp
-  static_assert(TZ % 32 == 0, "an output warp covers 32 cells of one tile row");
+  static_assert(TZ % 4 == 0, "tile rows start on 16-byte boundaries");
   static_assert(RP <= 32, "one producer lane per buffered row");
-  // collide lanes walk every buffered cell (row pitch W), so the 32 cells of
-  // a warp access are consecutive in shared memory: no bank conflicts
-  static_assert(32 * NCW * CPL >= RP * W, "CPL buffered cells per collide lane and plane");
+  static_assert(CPO == 1 ? NOW == TY && TZ == 32
+                         : TY == 1 && OZ == 32 * NOW && TZ <= 2 * OZ,
+                "the output lanes' cells cover the tile");
 };
 
 // Barriers and flags of a block, after the slots and the staging rows.
+template <int Q>
 struct TileSync {
-  uint64_t full[kMaxTileSlots];      // plane landed (producer arrive + copy bytes)
-  uint64_t collided[kMaxTileSlots];  // plane collided (one arrive per collide warp)
-  uint64_t consumed[kMaxTileSlots];  // plane read for the last time (one per output warp)
-  int abort;                      // a wait gave up
-  uint32_t issued;                // planes copied by the producer
-  uint32_t landed;                // planes a collide warp has seen land
+  static constexpr int S = Sweep<Q>::SLOTS;
+  uint64_t full[S];      // plane landed (producer arrive + copy bytes)
+  uint64_t collided[S];  // plane collided (one arrive per collide warp)
+  uint64_t consumed[S];  // plane read for the last time (one per output warp)
+  uint32_t wall[S][2 * TileShape<Q>::NCW];  // wall bits of the collided cells
+  int abort;             // a wait gave up
+  uint32_t issued;       // planes copied by the producer
 };
 
 template <int Q, int MODE>
 __host__ __device__ constexpr size_t tiled_stage_bytes() {
-  return MODE == kOutAoS ? static_cast<size_t>(TileShape<Q>::NOW) * 2 * 32 * Q * 4 : 0;
+  return MODE == kOutAoS
+             ? static_cast<size_t>(TileShape<Q>::NOW) * 32 * TileShape<Q>::CPO * Q * 4
+             : 0;
 }
 template <int Q, int MODE>
 __host__ __device__ constexpr size_t tiled_smem_bytes() {
-  return static_cast<size_t>(Sweep<Q>::SLOTS) * TileShape<Q>::PLANE * 4 + tiled_stage_bytes<Q, MODE>() +
-         sizeof(TileSync);
+  return static_cast<size_t>(Sweep<Q>::SLOTS) * TileShape<Q>::PLANE * 4 +
+         tiled_stage_bytes<Q, MODE>() + sizeof(TileSync<Q>);
 }
 
 // Host-computed geometry of the sweep.
@@ -163,8 +186,8 @@ __device__ __forceinline__ uint32_t plane_s(const TileGeo& t, const PlaneRef& p)
 }
 
 // Producer warp: lane 0 arms `bar` with the bytes of one plane (tile rows with
-// their halo), then lane rr copies buffered row rr into buf, so the copies of a
-// plane are issued together rather than one after another.
+// their halo cells), then lane rr copies buffered row rr into buf, so the
+// copies of a plane are issued together rather than one after another.
 template <int Q>
 __device__ __forceinline__ void tiled_issue(const StepArgs& a, const TileGeo& t,
                                             const PlaneRef& p, float* buf, uint64_t* bar,
@@ -172,30 +195,22 @@ __device__ __forceinline__ void tiled_issue(const StepArgs& a, const TileGeo& t,
   using T = TileShape<Q>;
   const uint32_t ps = plane_s(t, p);
   const uint32_t nrow = p.tyv + 2 * T::HR;
-  constexpr uint32_t cellb = Q * 4;
-  if (lane == 0) mbar_arrive_expect_tx(bar, nrow * (p.tzv + 2 * kTileHalo) * cellb);
+  if (lane == 0) mbar_arrive_expect_tx(bar, nrow * (p.tzv * Q + 2 * T::LCH) * 4);
   __syncwarp();
   const uint32_t rr = lane;
   if (t.no_copy || rr >= nrow) return;
-  const float* f = static_cast<const float*>(a.f_in);
   const uint32_t n2 = a.g.n2;
   const uint32_t r = wrapu(static_cast<int>(p.y0 + rr) - T::HR, t.NR);
-  const size_t rowc = static_cast<size_t>(ps) * t.SS + static_cast<size_t>(r) * t.SR;
-  float* dst = buf + static_cast<size_t>(rr) * T::W * Q;
-  uint32_t col = 0;  // buffer cell of the next copy
-  uint32_t z = p.z0 - kTileHalo;
-  if (p.z0 == 0) {  // left halo group wraps to the end of the row
-    bulk_copy_g2s(dst, f + (rowc + n2 - kTileHalo) * Q, kTileHalo * cellb, bar);
-    col = kTileHalo;
-    z = 0;
-  }
-  const bool wrap_r = p.z0 + p.tzv == n2;
-  const uint32_t zend = wrap_r ? n2 : p.z0 + p.tzv + kTileHalo;
-  bulk_copy_g2s(dst + static_cast<size_t>(col) * Q, f + (rowc + z) * Q, (zend - z) * cellb,
-                bar);
-  if (wrap_r)  // right halo group wraps to the start of the row
-    bulk_copy_g2s(dst + static_cast<size_t>(kTileHalo + p.tzv) * Q, f + rowc * Q,
-                  kTileHalo * cellb, bar);
+  const float* row = static_cast<const float*>(a.f_in) +
+                     (static_cast<size_t>(ps) * t.SS + static_cast<size_t>(r) * t.SR) * Q;
+  float* dst = buf + static_cast<size_t>(rr) * T::RW;
+  // words [b, e) of the row around the tile; either end may wrap
+  const bool wrap_l = p.z0 == 0, wrap_r = p.z0 + p.tzv == n2;
+  const uint32_t b = p.z0 * Q - (wrap_l ? 0u : T::LCH);
+  const uint32_t e = (p.z0 + p.tzv) * Q + (wrap_r ? 0u : T::LCH);
+  if (wrap_l) bulk_copy_g2s(dst, row + n2 * Q - T::LCH, T::LCH * 4, bar);
+  bulk_copy_g2s(dst + (wrap_l ? T::LCH : 0), row + b, (e - b) * 4, bar);
+  if (wrap_r) bulk_copy_g2s(dst + T::LCH + p.tzv * Q, row, T::LCH * 4, bar);
 }
 
 // p = C(f) of the reference state of cell c (k_prepare's arithmetic), with the
@@ -215,6 +230,51 @@ __device__ __forceinline__ void collide_ref(const StepArgs& a, uint32_t c, float
     const uint32_t seed = sr_seed(c, m.u[0], m.u[1], m.u[2], m.rd);
 #pragma unroll
     for (int q = 0; q < Q; ++q) d[q] = to_r(sr_one<S>(d[q], sr_bits(seed, d[q])));
+  }
+}
+
+// Wall-node swap of a lane's two cells (w0, w1: it is a wall cell).
+template <int Q>
+__device__ __forceinline__ void wall_swap2(F2 (&d)[Q], bool w0, bool w1) {
+#pragma unroll
+  for (int q = 1; q < Q; ++q) {
+    const int o = Lat<Q>::opp(q);
+    if (q > o) continue;
+    const F2 x = d[q], y = d[o];
+    d[q] = F2(w0 ? y.v.x : x.v.x, w1 ? y.v.y : x.v.y);
+    d[o] = F2(w0 ? x.v.x : y.v.x, w1 ? x.v.y : y.v.y);
+  }
+}
+
+// collide_ref for the two cells of a lane (c0, c1), two-wide arithmetic.
+template <int Q, class S, bool FORCE>
+__device__ __forceinline__ void collide_ref2(const StepArgs& a, uint32_t c0, uint32_t c1,
+                                             F2 (&d)[Q]) {
+  F2 F[3] = {0, 0, 0};
+  if (FORCE) {
+    float G0[3], G1[3];
+    if (a.force_mode == 2) {
+      load_force<Q, float>(a.force_field, c0, G0);
+      load_force<Q, float>(a.force_field, c1, G1);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) F[k] = F2(G0[k], G1[k]);
+    } else {
+      uniform_force<Q, float>(a, G0);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) F[k] = F2(G0[k]);
+    }
+  }
+  const Mom<F2> m = moments<Q, F2, FORCE>(d, F, true);
+  collide<Q, F2, FORCE>(d, m, F, F2(a.omega), F2(a.guo_c));
+  if constexpr (sizeof(S) == 2) {
+    const uint32_t s2 =
+        sr_pair(sr_seed(c0, m.u[0].v.x, m.u[1].v.x, m.u[2].v.x, m.rd.v.x),
+                sr_seed(c1, m.u[0].v.y, m.u[1].v.y, m.u[2].v.y, m.rd.v.y));
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const uint32_t w = sr_two<S>(d[q].v.x, d[q].v.y, s2);
+      d[q] = F2(PairT<S>::lo(w), PairT<S>::hi(w));
+    }
   }
 }
 
@@ -261,44 +321,37 @@ __device__ __forceinline__ void face_zero_gradient_ref(float (&d)[Q], const Step
   }
 }
 
-// Wall swap and faces of a pulled cell (apply_bc with the zero-gradient
-// neighbour taken from the reference state).  The swap is a select on every
-// pair and the faces are entered only when a cell of the warp lies on one:
-// fewer branches in the output warps' path than apply_bc's.
-template <int Q, class S, bool FACES, bool FORCE>
-__device__ __forceinline__ void apply_bc_ref(const StepArgs& a, const Cell& x, bool wall,
-                                             float (&d)[Q]) {
+// Faces `on` of a cell: inlet, then outlet, the zero-gradient neighbour taken
+// from the reference state.
+template <int Q, class S, bool FORCE>
+__device__ __forceinline__ void faces_ref(const StepArgs& a, const Cell& x, uint32_t on,
+                                          float (&d)[Q]) {
 #pragma unroll
-  for (int q = 1; q < Q; ++q) {
-    if (q < Lat<Q>::opp(q)) {
-      const float u = d[q], v = d[Lat<Q>::opp(q)];
-      d[q] = wall ? v : u;
-      d[Lat<Q>::opp(q)] = wall ? u : v;
-    }
-  }
-  if constexpr (FACES) {
-    const Geo& g = a.g;
-    uint32_t on = 0;
-#pragma unroll
-    for (int fi = 0; fi < 2; ++fi) {
-      const FaceK& fc = a.face[fi];
-      const uint32_t coord = fc.axis == 0 ? x.i0 : (fc.axis == 1 ? x.i1 : x.k);
-      const uint32_t nax = fc.axis == 0 ? g.n0 : (fc.axis == 1 ? g.n1 : g.n2);
-      if (fc.kind != kFaceNone && coord == (fc.side == 0 ? 0u : nax - 1)) on |= 1u << fi;
-    }
-    if (wall) on = 0;
-    if (__any_sync(__activemask(), on != 0)) {
-#pragma unroll
-      for (int fi = 0; fi < 2; ++fi) {
-        if (!((on >> fi) & 1u)) continue;
-        const FaceK& fc = a.face[fi];
-        if (fc.kind == kFacePressure) face_pressure<Q, float>(d, a, fi);
-        else if (fc.kind == kFaceVelocity) face_velocity<Q, float>(d, a, fi);
-        else face_zero_gradient_ref<Q, S, FORCE>(d, a, fi, x);
-      }
-    }
+  for (int fi = 0; fi < 2; ++fi) {
+    if (!((on >> fi) & 1u)) continue;
+    const FaceK& fc = a.face[fi];
+    if (fc.kind == kFacePressure) face_pressure<Q, float>(d, a, fi);
+    else if (fc.kind == kFaceVelocity) face_velocity<Q, float>(d, a, fi);
+    else face_zero_gradient_ref<Q, S, FORCE>(d, a, fi, x);
   }
 }
+// ... of one of a lane's two cells (HI: the high half).
+template <int Q, class S, bool FORCE, bool HI>
+__device__ __forceinline__ void faces_ref2(const StepArgs& a, const Cell& x, uint32_t on,
+                                           F2 (&d)[Q]) {
+  float t[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) t[q] = HI ? d[q].v.y : d[q].v.x;
+  faces_ref<Q, S, FORCE>(a, x, on, t);
+#pragma unroll
+  for (int q = 0; q < Q; ++q) d[q] = HI ? F2(d[q].v.x, t[q]) : F2(t[q], d[q].v.y);
+}
+
+// Cell J of a lane's one or two cells.
+template <int J>
+__device__ __forceinline__ float cell_of(float v) { return v; }
+template <int J>
+__device__ __forceinline__ float cell_of(F2 v) { return J == 0 ? v.v.x : v.v.y; }
 
 // A wall byte, loaded where the source places it: the output warps fetch the
 // next plane's byte one plane ahead, and a volatile load is neither moved
@@ -335,23 +388,34 @@ __device__ __forceinline__ bool mbar_try_wait_sleep(uint64_t* bar, uint32_t pari
 
 // Wait bounded by wall time (limit_ns of the global timer) that also ends when
 // another warp of the block has given up (*abort set); a wait that runs out
-// sets *abort itself.  Between polls the warp sleeps, up to max_sleep_ns, so
-// that waiting warps leave the issue slots to the working ones.
+// sets *abort itself.  Between polls the warp is suspended by the barrier's own
+// wait, so it takes few issue slots.
 __device__ __forceinline__ bool tile_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns,
-                                          volatile int* abort, uint32_t max_sleep_ns) {
+                                          volatile int* abort) {
   if (mbar_try_wait_sleep(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
-  uint32_t sleep = 32;
   for (;;) {
-    if (mbar_try_wait_sleep(bar, parity)) return true;
+#pragma unroll 1
+    for (int i = 0; i < 8; ++i)
+      if (mbar_try_wait_sleep(bar, parity)) return true;
     if (*abort) return false;
     if (globaltimer_ns() - t0 > limit_ns) break;
-    __nanosleep(sleep);
-    sleep = sleep < max_sleep_ns ? 2 * sleep : max_sleep_ns;
   }
   *abort = 1;
   return false;
 }
+
+// Place of the current plane in the ring: slot and parity of its barriers.
+template <int Q>
+struct Ring {
+  uint32_t s = 0, par = 0;
+  __device__ __forceinline__ void next() {
+    if (++s == static_cast<uint32_t>(Sweep<Q>::SLOTS)) {
+      s = 0;
+      par ^= 1u;
+    }
+  }
+};
 
 template <int Q, class S, int MODE, bool FACES, bool FORCE>
 __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
@@ -360,11 +424,11 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
   using R = float;
   static_assert(MODE == kOutAoS || MODE == kOutState, "f_bc out or the next state out");
   constexpr uint32_t S_ = Sweep<Q>::SLOTS;
-  static_assert(Sweep<Q>::SLOTS >= 5 && Sweep<Q>::SLOTS <= kMaxTileSlots, "ring depth");
+  static_assert(Sweep<Q>::SLOTS >= 5, "ring depth: three planes read, one collided, one landing");
   extern __shared__ __align__(128) unsigned char smem[];
   float* planes = reinterpret_cast<float*>(smem);
   float* stage = planes + static_cast<size_t>(S_) * T::PLANE;
-  TileSync* sync = reinterpret_cast<TileSync*>(
+  TileSync<Q>* sync = reinterpret_cast<TileSync<Q>*>(
       smem + static_cast<size_t>(S_) * T::PLANE * 4 + tiled_stage_bytes<Q, MODE>());
   volatile int* abort = &sync->abort;
   const Geo& g = a.g;
@@ -379,194 +443,287 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
     }
     sync->abort = 0;
     sync->issued = 0;
-    sync->landed = 0;
     fence_mbar_init();
   }
   __syncthreads();
 
   if (warp == 0) {
-    // ---- producer: copy plane P into slot P % S once plane P - S is consumed
-    {
-      PlaneRef L;
-      plane_first<Q>(a, t, blockIdx.x, L);
-      uint32_t P = 0;
-      for (; L.item < t.items; plane_next<Q>(a, t, L), ++P) {
-        const uint32_t sl = P % S_;
-        const bool ok = P < S_ ||
-                        tile_wait(&sync->consumed[sl], (P / S_ - 1) & 1u, t.wait_ns, abort, 1024);
-        if (!__all_sync(0xffffffffu, ok)) break;
-        fence_proxy_async_smem();
-        tiled_issue<Q>(a, t, L, planes + static_cast<size_t>(sl) * T::PLANE, &sync->full[sl],
-                       lane);
-      }
-      if (lane == 0) sync->issued = P;
+    // ---- producer: copy plane P into its slot once the slot's last plane is consumed
+    PlaneRef L;
+    plane_first<Q>(a, t, blockIdx.x, L);
+    Ring<Q> r;
+    uint32_t P = 0;
+    for (; L.item < t.items; plane_next<Q>(a, t, L), ++P, r.next()) {
+      const bool ok =
+          P < S_ || tile_wait(&sync->consumed[r.s], r.par ^ 1u, t.wait_ns, abort);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      fence_proxy_async_smem();
+      tiled_issue<Q>(a, t, L, planes + static_cast<size_t>(r.s) * T::PLANE, &sync->full[r.s],
+                     lane);
     }
+    if (lane == 0) sync->issued = P;
   } else if (warp <= static_cast<uint32_t>(T::NCW)) {
-    // ---- collide warps: plane P in place once it has landed; lane cells
-    // m_k = lane + 32 (warp - 1 + k NCW), k < CPL, of the buffered cells (row
-    // pitch W; the collided ones are columns kTileHalo - 1 .. kTileHalo + TZ),
-    // their loads issued together
-    using T2 = TileShape<Q>;
-    uint32_t soff[T2::CPL], rr[T2::CPL], cc[T2::CPL], rz[T2::CPL];
-    bool mine[T2::CPL];
+    // ---- collide warps: plane P in place once it has landed, two cells per
+    // lane; the wall bits of its cells go to the plane's words
+    const uint32_t j = warp - 1;
+    uint32_t rr[2], cc[2], soff[2], rz[2];
+    bool mine[2];
 #pragma unroll
-    for (int k = 0; k < T2::CPL; ++k) {
-      const uint32_t m = (warp - 1 + k * T2::NCW) * 32 + lane;
-      rr[k] = m / T::W;
-      cc[k] = m % T::W - (kTileHalo - 1);  // wraps above CW for the unused columns
-      soff[k] = m * Q;                      // its place in a slot
+    for (int k = 0; k < 2; ++k) {
+      const uint32_t m = (2 * j + k) * 32 + lane;
+      rr[k] = m / T::CW;
+      cc[k] = m % T::CW;
       mine[k] = false;
-      rz[k] = 0;
+      soff[k] = rz[k] = 0;
     }
     PlaneRef C;
     plane_first<Q>(a, t, blockIdx.x, C);
-    uint32_t P = 0, item = ~0u;
-    for (; C.item < t.items; plane_next<Q>(a, t, C), ++P) {
+    Ring<Q> r;
+    uint32_t item = ~0u;
+    for (; C.item < t.items; plane_next<Q>(a, t, C), r.next()) {
       if (C.item != item) {  // a new work item: the lane cells' rows and columns
         item = C.item;
 #pragma unroll
-        for (int k = 0; k < T2::CPL; ++k) {
+        for (int k = 0; k < 2; ++k) {
           mine[k] = rr[k] < C.tyv + 2 * T::HR && cc[k] < C.tzv + 2;
-          rz[k] = wrapu(static_cast<int>(C.y0 + rr[k]) - T::HR, t.NR) * t.SR +
-                  wrapu(static_cast<int>(C.z0 + cc[k]) - 1, g.n2);
+          // a lane without a cell runs the plane's first one and stores nothing
+          const uint32_t ry = mine[k] ? rr[k] : 0u, cz = mine[k] ? cc[k] : 0u;
+          soff[k] = ry * T::RW + (T::LCH - Q) + cz * Q;
+          rz[k] = wrapu(static_cast<int>(C.y0 + ry) - T::HR, t.NR) * t.SR +
+                  wrapu(static_cast<int>(C.z0 + cz) - 1, g.n2);
         }
       }
-      const uint32_t sl = P % S_;
-      const bool ok = tile_wait(&sync->full[sl], (P / S_) & 1u, t.wait_ns, abort, 1024);
-      if (!__all_sync(0xffffffffu, ok)) break;
-      if (lane == 0) atomicMax(&sync->landed, P + 1);
-      float* slot = planes + static_cast<size_t>(sl) * T::PLANE;
       const uint32_t cs0 = plane_s(t, C) * t.SS;
-      R d[T2::CPL][Q];
-#pragma unroll
-      for (int k = 0; k < T2::CPL; ++k) {
-        if (mine[k]) {
-#pragma unroll
-          for (int q = 0; q < Q; ++q) d[k][q] = to_offset<Q, R>(slot[soff[k] + q], q);
-        }
+      uint8_t wb[2] = {0, 0};
+      if (a.wall != nullptr) {  // fetched ahead of the wait for the plane
+        wb[0] = ld_wall(a.wall + cs0 + rz[0]);
+        wb[1] = ld_wall(a.wall + cs0 + rz[1]);
       }
+      const bool ok = tile_wait(&sync->full[r.s], r.par, t.wait_ns, abort);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      float* slot = planes + static_cast<size_t>(r.s) * T::PLANE;
+      // No branch around this body: given one per cell, the compiler splits it
+      // by which cells a lane owns and a warp runs it up to three times.
+      F2 d[Q];
 #pragma unroll
-      for (int k = 0; k < T2::CPL; ++k) {
-        if (mine[k]) {
-          collide_ref<Q, S, FORCE>(a, cs0 + rz[k], d[k]);
+      for (int q = 0; q < Q; ++q) d[q] = F2(slot[soff[0] + q], slot[soff[1] + q]);
 #pragma unroll
-          for (int q = 0; q < Q; ++q) slot[soff[k] + q] = d[k][q];
-        }
+      for (int q = 0; q < Q; ++q) d[q] = to_offset<Q, F2>(d[q], q);
+      collide_ref2<Q, S, FORCE>(a, cs0 + rz[0], cs0 + rz[1], d);
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        if (mine[0]) slot[soff[0] + q] = d[q].v.x;
+        if (mine[1]) slot[soff[1] + q] = d[q].v.y;
       }
+      const uint32_t w0 = __ballot_sync(0xffffffffu, wb[0] != 0);
+      const uint32_t w1 = __ballot_sync(0xffffffffu, wb[1] != 0);
       fence_proxy_async_smem();  // before the slot is refilled by a copy
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sync->collided[sl]);
+      if (lane == 0) {
+        sync->wall[r.s][2 * j] = w0;
+        sync->wall[r.s][2 * j + 1] = w1;
+        mbar_arrive(&sync->collided[r.s]);
+      }
     }
   } else {
-    // ---- output warps: tile row `ty` of plane P once P + 1 is collided
+    // ---- output warps: plane P once P + 1 is collided; one cell (ty, tz) per
+    // lane, or two (tz and tz + OZ)
+    constexpr bool kTwo = T::CPO == 2;
+    using V = typename std::conditional<kTwo, F2, float>::type;
+    constexpr int kSA = Lat<Q>::D == 3 ? 0 : 1;  // the internal axis of the sweep
     const uint32_t ow = warp - 1 - T::NCW;
-    const uint32_t ty = ow / (T::TZ / 32), tz = (ow % (T::TZ / 32)) * 32 + lane;
-    // this warp's two staging rows, used in turn: a plane's store may still be
-    // reading one while the next plane is staged in the other
-    float* const wst2 = stage + static_cast<size_t>(ow) * 2 * 32 * Q;
-    uint32_t nstore = 0;  // bulk stores this warp has issued
-    const uint32_t off = ((ty + T::HR) * T::W + kTileHalo + tz) * Q;  // own cell in a slot
+    const uint32_t ty = kTwo ? 0u : ow, tz = (kTwo ? ow * 32 : 0u) + lane;
+    float* const wst = stage + static_cast<size_t>(ow) * 32 * T::CPO * Q;  // staging rows
+    // the places of its cells among the collided ones (wall bits)
+    const uint32_t m0 = (ty + T::HR) * T::CW + tz + 1, m1 = m0 + T::OZ;
+    bool act0 = false, act1 = false;  // its cells lie inside the lattice
+    uint32_t off = 0, off1 = 0, col = 0, face0 = 0, face1 = 0;
+    Cell x{};
     PlaneRef O;
     plane_first<Q>(a, t, blockIdx.x, O);
-    uint32_t P = 0;
-    uint32_t wnext_c = ~0u;  // cell whose wall byte was fetched one plane ahead
-    uint8_t wnext = 0;
-    for (; O.item < t.items; plane_next<Q>(a, t, O), ++P) {
-      if (O.j < 1 || O.j > O.nv) continue;
-      const uint32_t sn = (P + 1) % S_;
-      const bool ok =
-          tile_wait(&sync->collided[sn], ((P + 1) / S_) & 1u, t.wait_ns, abort, 64);
-      if (!__all_sync(0xffffffffu, ok)) break;
-      const uint32_t ps = plane_s(t, O);
-      const bool act = ty < O.tyv && tz < O.tzv;
-      Cell x;
-      if (Lat<Q>::D == 3) {
-        x.i0 = ps;
-        x.i1 = O.y0 + ty;
-      } else {
-        x.i0 = 0;
-        x.i1 = ps;
-      }
-      x.k = O.z0 + tz;
-      x.c = ps * t.SS + (O.y0 + ty) * t.SR + x.k;
-      x.row = x.c - x.k;
-      x.srow = x.row;
-      float* const wst = wst2 + (nstore & 1u) * 32 * Q;
-      if constexpr (MODE == kOutAoS) {
-        // the store before the last one has finished reading this staging row
-        if (lane == 0) bulk_wait_read_1();
-        __syncwarp();
-      }
-      uint8_t wb = 0;
-      if (act && a.wall != nullptr) {
-        wb = x.c == wnext_c ? wnext : ld_wall(a.wall + x.c);
-        if (O.j < O.nv) {  // the same lane's cell of the next plane of this item
-          wnext_c = x.c + t.SS;
-          wnext = ld_wall(a.wall + wnext_c);
+    Ring<Q> r, rn;  // plane P, plane P + 1
+    rn.next();
+    uint32_t sm = S_ - 1;  // slot of plane P - 1
+    uint32_t item = ~0u;
+    for (; O.item < t.items; plane_next<Q>(a, t, O), sm = r.s, r.next(), rn.next()) {
+      if (O.item != item) {  // a new work item: the lane cells' column
+        item = O.item;
+        act0 = ty < O.tyv && tz < O.tzv;
+        act1 = kTwo && act0 && tz + T::OZ < O.tzv;
+        // A lane without a first cell runs the tile's first one, a lane without a
+        // second cell its first one again; neither stores it (no branch around
+        // the body, as above).
+        const uint32_t tye = act0 ? ty : 0u, tze = act0 ? tz : 0u;
+        off = ((tye + T::HR) * T::RW + T::LCH) + tze * Q;
+        off1 = act1 ? T::OZ * Q : 0u;
+        x.i1 = O.y0 + tye;  // D3Q19; the sweep's own coordinate with D2Q9
+        x.k = O.z0 + tze;
+        col = (O.y0 + tye) * t.SR + x.k;
+        // faces along the axes across the sweep
+        face0 = face1 = 0;
+        if constexpr (FACES) {
+#pragma unroll
+          for (int fi = 0; fi < 2; ++fi) {
+            const FaceK& fc = a.face[fi];
+            if (fc.kind == kFaceNone || fc.axis == kSA) continue;
+            const uint32_t last = (fc.axis == 1 ? g.n1 : g.n2) - 1;
+            const uint32_t at = fc.side == 0 ? 0u : last;
+            if (act0 && (fc.axis == 1 ? x.i1 : x.k) == at) face0 |= 1u << fi;
+            if (act1 && x.k + T::OZ == at) face1 |= 1u << fi;
+          }
         }
       }
-      R d[Q];
-      R F[3] = {0, 0, 0};
-      Mom<R> mo;
-      const bool wall = wb != 0;
-      if (act) {
+      if (O.j < 1 || O.j > O.nv) continue;
+      const bool ok = tile_wait(&sync->collided[rn.s], rn.par, t.wait_ns, abort);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      const uint32_t ps = plane_s(t, O);
+      if (Lat<Q>::D == 3) x.i0 = ps;
+      else x.i1 = ps;
+      x.c = ps * t.SS + col;
+      x.row = x.c - x.k;
+      x.srow = x.row;
+      const uint32_t* wbits = sync->wall[r.s];
+      const bool wall0 = act0 && ((wbits[m0 >> 5] >> (m0 & 31u)) & 1u) != 0;
+      const bool wall1 = act1 && ((wbits[m1 >> 5] >> (m1 & 31u)) & 1u) != 0;
+      V d[Q];
+      {
         // the three planes of the pull: x - e_q lies in plane P - c_s(q)
-        const float* pm = planes + static_cast<size_t>((P + S_ - 1) % S_) * T::PLANE + off;
-        const float* p0 = planes + static_cast<size_t>(P % S_) * T::PLANE + off;
-        const float* pp = planes + static_cast<size_t>(sn) * T::PLANE + off;
+        const float* pm = planes + static_cast<size_t>(sm) * T::PLANE + off;
+        const float* p0 = planes + static_cast<size_t>(r.s) * T::PLANE + off;
+        const float* pp = planes + static_cast<size_t>(rn.s) * T::PLANE + off;
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
           const int cs = Sweep<Q>::cs(q);
-          const float* base = cs > 0 ? pm : (cs < 0 ? pp : p0);
-          d[q] = base[(-Sweep<Q>::cr(q) * T::W - Lat<Q>::c2(q)) * Q + q];
-        }
-        if (FORCE) {
-          if (a.force_mode == 2) load_force<Q, float>(a.force_field, x.c, F);
-          else uniform_force<Q, R>(a, F);
-        }
-        apply_bc_ref<Q, S, FACES, FORCE>(a, x, wall, d);
-        mo = moments<Q, R, FORCE>(d, F, true);
-        if constexpr (MODE == kOutAoS) {
-          float* row = wst + lane * Q;
-#pragma unroll
-          for (int q = 0; q < Q; ++q) row[q] = from_offset<Q, R>(d[q], q);
+          const float* base = (cs > 0 ? pm : (cs < 0 ? pp : p0)) +
+                              (-Sweep<Q>::cr(q) * T::RW - Lat<Q>::c2(q) * Q + q);
+          if constexpr (kTwo) d[q] = F2(base[0], base[off1]);
+          else d[q] = base[0];
         }
       }
+      V F[3] = {0, 0, 0};
+      if (FORCE) {
+        float G0[3], G1[3];
+        if (a.force_mode == 2) {
+          load_force<Q, float>(a.force_field, x.c, G0);
+          if constexpr (kTwo)
+            load_force<Q, float>(a.force_field, act1 ? x.c + T::OZ : x.c, G1);
+        } else {
+          uniform_force<Q, R>(a, G0);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) G1[k] = G0[k];
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          if constexpr (kTwo) F[k] = F2(G0[k], G1[k]);
+          else F[k] = G0[k];
+        }
+      }
+      // obstacles are clustered: most warps hold no wall cell
+      if (__any_sync(0xffffffffu, wall0 || wall1)) {
+        if constexpr (kTwo) {
+          wall_swap2<Q>(d, wall0, wall1);
+        } else {
+#pragma unroll
+          for (int q = 1; q < Q; ++q) {
+            const int o = Lat<Q>::opp(q);
+            if (q > o) continue;
+            const float u = d[q], v = d[o];
+            d[q] = wall0 ? v : u;
+            d[o] = wall0 ? u : v;
+          }
+        }
+      }
+      if constexpr (FACES) {
+        uint32_t on0 = face0, on1 = face1;
+#pragma unroll
+        for (int fi = 0; fi < 2; ++fi) {
+          const FaceK& fc = a.face[fi];
+          if (fc.kind != kFaceNone && fc.axis == kSA && ps == (fc.side == 0 ? 0u : t.NS - 1)) {
+            on0 |= 1u << fi;
+            on1 |= 1u << fi;
+          }
+        }
+        if (__any_sync(0xffffffffu, (on0 | on1) != 0)) {
+          // wall face cells keep the swapped populations
+          if constexpr (kTwo) {
+            Cell x1 = x;
+            x1.k += T::OZ;
+            if (act0 && !wall0 && on0) faces_ref2<Q, S, FORCE, false>(a, x, on0, d);
+            if (act1 && !wall1 && on1) faces_ref2<Q, S, FORCE, true>(a, x1, on1, d);
+          } else if (act0 && !wall0 && on0) {
+            faces_ref<Q, S, FORCE>(a, x, on0, d);
+          }
+          __syncwarp();
+        }
+      }
+      const Mom<V> mo = moments<Q, V, FORCE>(d, F, true);
       if constexpr (MODE == kOutAoS) {
-        // The warp's cells are a prefix of one contiguous run of the output.
-        // The proxy fence comes before this warp's global stores of the
+        // this warp's earlier store has read the staging rows
+        if (lane == 0) bulk_wait_read();
+        __syncwarp();
+        float* row = wst + lane * Q;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const V v = from_offset<Q, V>(d[q], q);
+          row[q] = cell_of<0>(v);
+          if constexpr (kTwo) row[32 * Q + q] = cell_of<1>(v);
+        }
+        // The warp's cells are prefixes of one or two contiguous runs of the
+        // output.  The proxy fence comes before this warp's global stores of the
         // moments, so that it waits only for the staging writes.
-        const uint32_t nvalid = __popc(__ballot_sync(0xffffffffu, act));
+        const uint32_t n0 = __popc(__ballot_sync(0xffffffffu, act0));
+        const uint32_t n1 = kTwo ? __popc(__ballot_sync(0xffffffffu, act1)) : 0u;
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0 && nvalid > 0)
-          bulk_store_s2g(static_cast<float*>(a.f_out) + static_cast<size_t>(x.c) * Q, wst,
-                         nvalid * Q * 4);
-        nstore += nvalid > 0 ? 1u : 0u;
+        if (lane == 0 && n0 > 0) {
+          float* out = static_cast<float*>(a.f_out) + static_cast<size_t>(x.c) * Q;
+          bulk_store2_s2g(out, wst, n0 * Q * 4, out + T::OZ * Q, wst + 32 * Q, n1 * Q * 4);
+        }
       }
-      if (act) {
-        store_moments<Q, float>(a, x.c, mo, wall);
-        if constexpr (MODE == kOutState) {
-          collide<Q, R, FORCE>(d, mo, F, static_cast<R>(a.omega), static_cast<R>(a.guo_c));
-          S* out = static_cast<S*>(a.pout) + x.srow + x.k;
-          if constexpr (sizeof(S) == 2) {
-            const uint32_t seed = sr_seed(x.c, mo.u[0], mo.u[1], mo.u[2], mo.rd);
+      if (act0) {
+        Mom<R> v0, v1;
+        v0.rd = cell_of<0>(mo.rd), v1.rd = cell_of<1>(mo.rd);
+        v0.rho = cell_of<0>(mo.rho), v1.rho = cell_of<1>(mo.rho);
 #pragma unroll
-            for (int q = 0; q < Q; ++q)
-              out[static_cast<uint32_t>(q) * g.pstride] = sr_one<S>(d[q], sr_bits(seed, d[q]));
+        for (int k = 0; k < 3; ++k) v0.u[k] = cell_of<0>(mo.u[k]), v1.u[k] = cell_of<1>(mo.u[k]);
+        store_moments<Q, float>(a, x.c, v0, wall0);
+        if (act1) store_moments<Q, float>(a, x.c + T::OZ, v1, wall1);
+        if constexpr (MODE == kOutState) {
+          collide<Q, V, FORCE>(d, mo, F, static_cast<V>(a.omega), static_cast<V>(a.guo_c));
+          S* out = static_cast<S*>(a.pout) + x.c;
+          if constexpr (sizeof(S) == 2) {
+            const uint32_t s2 = sr_pair(sr_seed(x.c, v0.u[0], v0.u[1], v0.u[2], v0.rd),
+                                        sr_seed(x.c + T::OZ, v1.u[0], v1.u[1], v1.u[2], v1.rd));
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+              S* o = out + static_cast<uint32_t>(q) * g.pstride;
+              if constexpr (kTwo) {
+                const uint32_t w = sr_two<S>(cell_of<0>(d[q]), cell_of<1>(d[q]), s2);
+                reinterpret_cast<unsigned short*>(o)[0] = static_cast<unsigned short>(w & 0xffffu);
+                if (act1)
+                  reinterpret_cast<unsigned short*>(o)[T::OZ] = static_cast<unsigned short>(w >> 16);
+              } else {
+                o[0] = sr_one<S>(d[q], sr_bits(s2, d[q]));
+              }
+            }
           } else {
 #pragma unroll
-            for (int q = 0; q < Q; ++q) out[static_cast<uint32_t>(q) * g.pstride] = d[q];
+            for (int q = 0; q < Q; ++q) {
+              S* o = out + static_cast<uint32_t>(q) * g.pstride;
+              o[0] = cell_of<0>(d[q]);
+              if (act1) o[T::OZ] = cell_of<1>(d[q]);
+            }
           }
         }
       }
       __syncwarp();
       if (lane == 0) {
         // plane P - 1 has had its last reader; at the end of an item, P and P + 1 too
-        mbar_arrive(&sync->consumed[(P + S_ - 1) % S_]);
+        mbar_arrive(&sync->consumed[sm]);
         if (O.j == O.nv) {
-          mbar_arrive(&sync->consumed[P % S_]);
-          mbar_arrive(&sync->consumed[sn]);
+          mbar_arrive(&sync->consumed[r.s]);
+          mbar_arrive(&sync->consumed[rn.s]);
         }
       }
     }
@@ -578,10 +735,11 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
   __syncthreads();
   if (tid == 0 && sync->abort) {
     atomicOr(a.status, 1);
-    // copies issued and not seen landing: wait for them (bounded) before exit
+    // the last copies issued may be in flight: wait for them (bounded) before exit
     sync->abort = 0;
-    for (uint32_t P = sync->landed; P < sync->issued; ++P)
-      if (!tile_wait(&sync->full[P % S_], (P / S_) & 1u, t.wait_ns, abort, 512)) break;
+    const uint32_t n = sync->issued;
+    for (uint32_t P = n > S_ ? n - S_ : 0; P < n; ++P)
+      if (!tile_wait(&sync->full[P % S_], (P / S_) & 1u, t.wait_ns, abort)) break;
   }
 }
 
