@@ -284,12 +284,15 @@ int lbm_pipe_rollout(const lbm_plan* plan, lbm_stream_t stream, const void* f_in
  * a checkpoint of the populations every `checkpoint_every` steps (<= 0: the
  * ceiling of sqrt(n_steps)) in the workspace, and the backward recomputes each
  * segment storing only (rho, u) per step, then runs the hand-written adjoint
- * step.  The workspace must stay untouched between the two calls. */
+ * step.  Where (rho, u) of every step take no more room than that (short
+ * rollouts, checkpoint_every >= n_steps), the forward keeps those instead and
+ * nothing is recomputed.  The workspace must stay untouched between the two
+ * calls. */
 int lbm_adjoint_workspace_bytes(const lbm_plan* plan, int64_t n_steps, int64_t checkpoint_every,
                                 size_t* bytes);
 
 /* Same result as lbm_rollout (f_out, moments of the last step), plus the
- * checkpoints the backward needs.  f_in must not alias f_out. */
+ * checkpoints or moments the backward needs.  f_in must not alias f_out. */
 int lbm_rollout_forward(const lbm_plan* plan, lbm_stream_t stream, const void* f_in, void* f_out,
                         int64_t n_steps, int64_t checkpoint_every, const lbm_step_args* args,
                         const lbm_moments* out, void* workspace, size_t workspace_bytes);

@@ -16,8 +16,11 @@
 //   G = omega b + d / rho,  h = omega a - G . u.
 // (From dfeq_q/df_r = w_q [P_q + grad P_q . (e_r - u)], du/df_r = (e_r - u)/rho,
 // du/dF = I/(2 rho); the Guo term depends on f only through u.)
-// The Jacobian needs only (rho^n, u^n, F): the recomputed forward stores them
-// (16 B per cell and step) instead of the populations.
+// The Jacobian needs only (rho^n, u^n, F), 16 B per cell and step, not the
+// populations.  Where the moments of every step fit into the room that
+// checkpoints and one segment's moments would take, the forward pass keeps them
+// and the backward pass recomputes nothing; longer rollouts checkpoint the
+// populations and recompute each segment's moments.
 // Adjoint populations are kept in f units (dL/df), one plane per direction.
 #pragma once
 
@@ -72,6 +75,9 @@ __global__ void __launch_bounds__(kBlock) k_adj_init(const AdjArgs a) {
   constexpr int D = Lat<Q>::D;
   constexpr int sh = 3 - D;
   const uint32_t c = blockIdx.x * kBlock + threadIdx.x;
+  const IO* gf = nullptr;  // this cell's dL/df, staged from the reference layout
+  if (a.g_f != nullptr)
+    gf = aos_fill<Q, IO>(static_cast<const IO*>(a.g_f), blockIdx.x * kBlock, a.g.ncell);
   if (c >= a.g.ncell) return;
   const bool wall = a.wall != nullptr && a.wall[c] != 0;
   const R rho = static_cast<R>(static_cast<const IO*>(a.rho)[c]);
@@ -93,7 +99,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_init(const AdjArgs a) {
     if (Lat<Q>::c0(q)) v += Lat<Q>::c0(q) > 0 ? gu[0] * inv : -gu[0] * inv;
     if (Lat<Q>::c1(q)) v += Lat<Q>::c1(q) > 0 ? gu[1] * inv : -gu[1] * inv;
     if (Lat<Q>::c2(q)) v += Lat<Q>::c2(q) > 0 ? gu[2] * inv : -gu[2] * inv;
-    if (a.g_f) v += static_cast<R>(static_cast<const IO*>(a.g_f)[static_cast<size_t>(c) * Q + q]);
+    if (gf != nullptr) v += static_cast<R>(gf[q]);
     lam[q] = v;
   }
   if (a.dF != nullptr) {
@@ -103,17 +109,15 @@ __global__ void __launch_bounds__(kBlock) k_adj_init(const AdjArgs a) {
   adj_store<Q, S>(a, c, lam, wall);
 }
 
-// One reverse step (see the header comment).  MODE kAdjOutAoS writes lambda^0
-// = dL/df^0 in the reference (grid, Q) layout instead of mu.
+// One reverse step of cell cidx (see the header comment).  MODE kAdjOutAoS puts
+// lambda^0 = dL/df^0 into the thread's row of the staging tile instead of mu.
 template <int Q, class S, bool FORCE, int MODE>
-__global__ void __launch_bounds__(kBlock, min_blocks<S>()) k_adj_step(const AdjArgs a) {
+__device__ __forceinline__ void adj_cell(const AdjArgs& a, uint32_t cidx) {
   using R = typename StoreT<S>::R;
   using IO = typename StoreT<S>::IO;
   constexpr int D = Lat<Q>::D;
   constexpr int sh = 3 - D;
   const Geo& g = a.g;
-  const uint32_t cidx = blockIdx.x * kBlock + threadIdx.x;
-  if (cidx >= g.ncell) return;
   const Cell x = locate(g, cidx);
 
   // nu_q = mu(x + e_q)_q: source rows at +e_q (periodic).
@@ -213,12 +217,23 @@ __global__ void __launch_bounds__(kBlock, min_blocks<S>()) k_adj_step(const AdjA
       p[d] += static_cast<double>(R(0.5) * G[d + sh] + cg * b[d + sh]);
   }
   if constexpr (MODE == kAdjOutAoS) {
-    IO* o = static_cast<IO*>(a.grad_f0) + static_cast<size_t>(cidx) * Q;
+    IO* o = aos_tile<Q, IO>() + threadIdx.x * Q;
 #pragma unroll
     for (int q = 0; q < Q; ++q) o[q] = static_cast<IO>(lam[q]);
   } else {
     adj_store<Q, S>(a, cidx, lam, wall);
   }
+}
+
+// The last reverse step writes the block's cells as one contiguous run: stored
+// per thread, 76 B apart, it took 88 us at 96^3 where the others took 28.
+template <int Q, class S, bool FORCE, int MODE>
+__global__ void __launch_bounds__(kBlock, min_blocks<S>()) k_adj_step(const AdjArgs a) {
+  using IO = typename StoreT<S>::IO;
+  const uint32_t cidx = blockIdx.x * kBlock + threadIdx.x;
+  if (cidx < a.g.ncell) adj_cell<Q, S, FORCE, MODE>(a, cidx);
+  if constexpr (MODE == kAdjOutAoS)
+    aos_flush<Q, IO>(static_cast<IO*>(a.grad_f0), blockIdx.x * kBlock, a.g.ncell);
 }
 
 // Sum of a (grid, D) FP64 field into out[0..D-1] (fixed order, two passes via

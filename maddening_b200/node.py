@@ -525,7 +525,10 @@ class LBMNode(SimulationNode):
         hand-written adjoint (``lbm_rollout_forward`` / ``lbm_rollout_backward``).
 
         Populations are checkpointed every ``checkpoint_every`` steps (0: the
-        ceiling of sqrt(n_steps)); the backward recomputes each segment.  Walls
+        ceiling of sqrt(n_steps)) and the backward recomputes each segment; where
+        the density and velocity of every step take no more memory than that (short
+        rollouts, or ``checkpoint_every >= n_steps``) they are kept instead and
+        nothing is recomputed.  Walls
         and body forces only (no face conditions); FP32 or FP64 storage.
         """
         if int(n_steps) < 1:
@@ -571,6 +574,7 @@ class _RolloutFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, f0, force, node, wall_state, bi, n_steps, checkpoint_every):
+        ctx.set_materialize_grads(False)  # an unused output needs no zeros (76 B per cell for f)
         dev = f0.device
         plan = node.plan
         D, grid = node._D, node._grid_shape
