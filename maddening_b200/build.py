@@ -17,6 +17,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -24,7 +25,8 @@ ROOT = PKG.parent
 CSRC = PKG / "csrc"
 LIB = PKG / "liblbm_b200.so"
 DIGEST = PKG / "liblbm_b200.so.sha256"
-SOURCES = ["lbm_abi.cu", "lbm_tiled.cu"]
+SOURCES = ["lbm_abi.cu", "lbm_steps.cu", "lbm_batch.cu", "lbm_tiled.cu", "lbm_grad.cu",
+           "lbm_pipe.cu"]
 HEADERS = ["lbm_host.h", "lbm_kernels.cuh", "lbm_lattice.cuh", "lbm_adjoint.cuh",
            "lbm_staged.cuh", "lbm_tiled.cuh", "lbm_pair.cuh", "lbm_pipe.cuh",
            "lbm_multiphase.cuh", "lbm_pack.cuh"]
@@ -32,12 +34,25 @@ HEADERS = ["lbm_host.h", "lbm_kernels.cuh", "lbm_lattice.cuh", "lbm_adjoint.cuh"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CFLAGS = ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
           "-Xcompiler", "-fPIC,-O3"]
-# A split compile is faster (two minutes instead of eight for lbm_abi.cu) but
-# its code differs from build to build, with the way the unit happens to be
-# divided: builds of one k_tiled source ran a 256^3 update in 0.62 or 0.68 ms,
-# and in 0.60 compiled whole.  The tiled kernels are compiled whole; the
-# others timed alike both ways.
-UNIT_FLAGS = {"lbm_abi.cu": ["--split-compile=0"]}
+# Units: (source, object name, definitions).  The step kernels are compiled once
+# per lattice and storage, side by side, and each unit as a whole: a split
+# compile of one large unit gave code that differed from build to build, with
+# the way the unit happened to be divided (builds of one k_tiled source ran a
+# 256^3 update in 0.62 or 0.68 ms, and in 0.60 compiled whole).
+_STORES = {"f32": "float", "f16": "__half", "bf16": "__nv_bfloat16", "f64": "double"}
+
+
+def units():
+    out = []
+    for src, stores in (("lbm_steps.cu", _STORES), ("lbm_batch.cu", _STORES),
+                        ("lbm_tiled.cu", ("f16", "bf16", "f32"))):
+        for q in (19, 9):
+            for st in stores:
+                out.append((src, f"{Path(src).stem}_{q}_{st}",
+                            [f"-DLBM_UNIT_Q={q}", f"-DLBM_UNIT_S={_STORES[st]}"]))
+    return out + [(s, Path(s).stem, []) for s in ("lbm_grad.cu", "lbm_pipe.cu", "lbm_abi.cu")]
+
+
 LFLAGS = ["-shared", "-cudart", "static"]
 
 
@@ -61,7 +76,7 @@ def input_digest() -> str:
         h.update(f.name.encode())
         h.update(f.read_bytes())
     h.update(" ".join(ARCH + CFLAGS + LFLAGS).encode())
-    h.update(repr(sorted(UNIT_FLAGS.items())).encode())
+    h.update(repr(units()).encode())
     try:
         h.update(subprocess.run([nvcc(), "--version"], capture_output=True,
                                 text=True).stdout.encode())
@@ -80,25 +95,29 @@ def build(verbose: bool = False, force: bool = False) -> Path:
     digest = input_digest()
     objdir = PKG / "_build"
     objdir.mkdir(exist_ok=True)
-    procs = []
-    for src in SOURCES:
-        obj = objdir / (Path(src).stem + ".o")
-        cmd = [nvcc(), *ARCH, *CFLAGS, *UNIT_FLAGS.get(src, []), "-I", str(ROOT / "include"),
-               "-c", str(CSRC / src), "-o", str(obj)]
+
+    def compile_unit(unit):
+        src, name, defs = unit
+        obj = objdir / (name + ".o")
+        cmd = [nvcc(), *ARCH, *CFLAGS, *defs, "-I", str(ROOT / "include"), "-c",
+               str(CSRC / src), "-o", str(obj)]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
-            print(" ".join(cmd), flush=True)
-        procs.append((obj, subprocess.Popen(cmd, stdout=subprocess.PIPE,
-                                            stderr=subprocess.STDOUT, text=True)))
+        res = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        return obj, " ".join(cmd), res
+
+    with ThreadPoolExecutor(max_workers=max(1, os.cpu_count() or 1)) as pool:
+        done = list(pool.map(compile_unit, units()))
     failed = False
-    for _obj, pr in procs:
-        out, _ = pr.communicate()
-        if verbose or pr.returncode != 0:
-            sys.stdout.write(out)
-        failed |= pr.returncode != 0
+    for _obj, cmd, res in done:
+        if verbose:
+            print(cmd, flush=True)
+        if verbose or res.returncode != 0:
+            sys.stdout.write(res.stdout)
+        failed |= res.returncode != 0
     if failed:
         raise RuntimeError("nvcc failed")
-    cmd = [nvcc(), *ARCH, *LFLAGS, *(str(o) for o, _ in procs), "-o", str(LIB) + ".tmp"]
+    cmd = [nvcc(), *ARCH, *LFLAGS, *(str(d[0]) for d in done), "-o", str(LIB) + ".tmp"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         sys.stderr.write(res.stdout + res.stderr)

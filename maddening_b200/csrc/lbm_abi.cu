@@ -11,14 +11,9 @@
 #include <vector>
 
 #include "../../include/lbm_b200.h"
-#include "lbm_adjoint.cuh"
-#include "lbm_kernels.cuh"
-#include "lbm_pair.cuh"
-#include "lbm_multiphase.cuh"
-#include "lbm_pack.cuh"
-#include "lbm_pipe.cuh"
-#include "lbm_staged.cuh"
 #include "lbm_host.h"
+#include "lbm_kernels.cuh"
+#include "lbm_pack.cuh"
 
 thread_local std::string g_last_error;
 
@@ -38,12 +33,6 @@ int cuda_check(cudaError_t e, const char* what) {
 }
 
 namespace {
-
-size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
-
-size_t state_bytes(const lbm_plan* p) {
-  return static_cast<size_t>(p->Q) * static_cast<size_t>(p->g.ncell) * p->elem;
-}
 
 // Multiply-high constants for x / d, 0 <= x < 2^31 (see lbm::fdiv).
 lbm::FastDiv make_fastdiv(uint32_t d) {
@@ -142,361 +131,6 @@ int build_args(const lbm_plan* p, const lbm_step_args* args, const lbm_moments* 
   return LBM_OK;
 }
 
-unsigned grid_for(uint64_t n) { return static_cast<unsigned>((n + lbm::kBlock - 1) / lbm::kBlock); }
-
-template <int Q, class S>
-int launch_prepare(const lbm::StepArgs& a, cudaStream_t s) {
-  const unsigned grid = grid_for(a.g.ncell);
-  if (a.force_mode != 0)
-    lbm::k_prepare<Q, S, true><<<grid, lbm::kBlock, 0, s>>>(a);
-  else
-    lbm::k_prepare<Q, S, false><<<grid, lbm::kBlock, 0, s>>>(a);
-  return cuda_check(cudaGetLastError(), "k_prepare launch");
-}
-
-template <int Q, class S, int MODE>
-void launch_step_mode(const lbm::StepArgs& a, cudaStream_t s) {
-  const unsigned grid = grid_for(a.cell_end - a.cell0);
-  const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
-  const bool force = a.force_mode != 0;
-  if (faces) {
-    if (force) lbm::k_step<Q, S, MODE, true, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step<Q, S, MODE, true, false><<<grid, lbm::kBlock, 0, s>>>(a);
-  } else {
-    if (force) lbm::k_step<Q, S, MODE, false, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step<Q, S, MODE, false, false><<<grid, lbm::kBlock, 0, s>>>(a);
-  }
-}
-
-template <int Q, class S>
-int launch_step(const lbm::StepArgs& a, bool final_aos, cudaStream_t s) {
-  if (final_aos) launch_step_mode<Q, S, lbm::kOutAoS>(a, s);
-  else launch_step_mode<Q, S, lbm::kOutState>(a, s);
-  return cuda_check(cudaGetLastError(), "k_step launch");
-}
-
-// Paired-cell state step (lbm_pair.cuh): the default for 16-bit storage,
-// opt-in for FP32 (LBM_PLAN_PAIRED_CELLS), off with LBM_PLAN_SINGLE_CELLS.
-// Rows of even length (row segments when they split into warps of 64 cells,
-// instance-wide pairs otherwise); state planes and the wall mask aligned for
-// the pair width.
-template <class S>
-bool pair_ok(const lbm_plan* p, const lbm::StepArgs& a) {
-  if constexpr (sizeof(S) == 8) {
-    return false;
-  } else {
-    if (p->flags & LBM_PLAN_SINGLE_CELLS) return false;
-    if (sizeof(S) == 4 && !(p->flags & LBM_PLAN_PAIRED_CELLS)) return false;
-    const uintptr_t al = 2 * sizeof(S);
-    return p->g.n2 % 2 == 0 && reinterpret_cast<uintptr_t>(a.pin) % al == 0 &&
-           reinterpret_cast<uintptr_t>(a.pout) % al == 0 &&
-           reinterpret_cast<uintptr_t>(a.wall) % 2 == 0;
-  }
-}
-
-template <int Q, class S, int W>
-void launch_pair_w(const lbm::StepArgs& a, cudaStream_t s) {
-  const dim3 grid(a.g.n0 * a.g.n1, a.g.n2 / (64 * W));
-  const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
-  const bool force = a.force_mode != 0;
-  if (faces) {
-    if (force) lbm::k_step_pair<Q, S, true, true, W><<<grid, 32 * W, 0, s>>>(a);
-    else lbm::k_step_pair<Q, S, true, false, W><<<grid, 32 * W, 0, s>>>(a);
-  } else {
-    if (force) lbm::k_step_pair<Q, S, false, true, W><<<grid, 32 * W, 0, s>>>(a);
-    else lbm::k_step_pair<Q, S, false, false, W><<<grid, 32 * W, 0, s>>>(a);
-  }
-}
-
-template <int Q, class S, int W>
-void launch_quad_w(const lbm::StepArgs& a, cudaStream_t s) {
-  const dim3 grid(a.g.n0 * a.g.n1, a.g.n2 / (128 * W));
-  const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
-  const bool force = a.force_mode != 0;
-  if (faces) {
-    if (force) lbm::k_step_quad<Q, S, true, true, W><<<grid, 32 * W, 0, s>>>(a);
-    else lbm::k_step_quad<Q, S, true, false, W><<<grid, 32 * W, 0, s>>>(a);
-  } else {
-    if (force) lbm::k_step_quad<Q, S, false, true, W><<<grid, 32 * W, 0, s>>>(a);
-    else lbm::k_step_quad<Q, S, false, false, W><<<grid, 32 * W, 0, s>>>(a);
-  }
-}
-
-// The four-cell form (16-bit storage): rows of a multiple of 128 cells,
-// unpadded state rows, 8-byte aligned planes and a 4-byte aligned wall mask.
-// D3Q19 also takes it (a B200 sweep at 256^3: 79.2k MLUPS FP16 against 71.7k
-// for pairs, at 20 resident warps and 96 registers) on rows of a multiple of
-// 256 cells: with one-warp blocks (rows of 128) it keeps 15 warps resident and
-// loses to pairs.
-#ifndef LBM_QUAD_Q19
-#define LBM_QUAD_Q19 1
-#endif
-template <int Q, class S>
-bool quad_ok(const lbm::StepArgs& a) {
-  return (Q == 9 || (LBM_QUAD_Q19 && Q == 19)) && sizeof(S) == 2 &&
-         a.g.n2 % (Q == 19 ? 256 : 128) == 0 && a.g.rstride == a.g.n2 &&
-         a.g.pstride % 4 == 0 && reinterpret_cast<uintptr_t>(a.pin) % 8 == 0 &&
-         reinterpret_cast<uintptr_t>(a.pout) % 8 == 0 &&
-         reinterpret_cast<uintptr_t>(a.wall) % 4 == 0;
-}
-
-template <int Q, class S>
-void launch_gquad(const lbm::StepArgs& a, cudaStream_t s) {
-  const unsigned grid = grid_for(a.g.ncell / 4);
-  const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
-  const bool force = a.force_mode != 0;
-  if (faces) {
-    if (force) lbm::k_step_gquad<Q, S, true, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step_gquad<Q, S, true, false><<<grid, lbm::kBlock, 0, s>>>(a);
-  } else {
-    if (force) lbm::k_step_gquad<Q, S, false, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step_gquad<Q, S, false, false><<<grid, lbm::kBlock, 0, s>>>(a);
-  }
-}
-
-// The instance-wide four-cell form: D2Q9 with 16-bit storage, rows of a
-// multiple of 4 cells (a quad never spans two rows), the same alignment as the
-// row form (4000^2 channel: 148.9k MLUPS against 114.4k for pairs).  D3Q19
-// keeps pairs there: with per-lane rows its 96-register budget spills and it
-// lost (48.3k against 61.9k at 160^3; 56.4k at 128 registers and 16 warps).
-template <int Q, class S>
-bool gquad_ok(const lbm::StepArgs& a) {
-  return Q == 9 && sizeof(S) == 2 && a.g.n2 % 4 == 0 &&
-         a.g.rstride == a.g.n2 && a.g.pstride % 4 == 0 &&
-         reinterpret_cast<uintptr_t>(a.pin) % 8 == 0 &&
-         reinterpret_cast<uintptr_t>(a.pout) % 8 == 0 &&
-         reinterpret_cast<uintptr_t>(a.wall) % 4 == 0;
-}
-
-template <int Q, class S>
-void launch_gpair(const lbm::StepArgs& a, cudaStream_t s) {
-  const unsigned grid = grid_for(a.g.ncell / 2);
-  const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
-  const bool force = a.force_mode != 0;
-  if (faces) {
-    if (force) lbm::k_step_gpair<Q, S, true, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step_gpair<Q, S, true, false><<<grid, lbm::kBlock, 0, s>>>(a);
-  } else {
-    if (force) lbm::k_step_gpair<Q, S, false, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step_gpair<Q, S, false, false><<<grid, lbm::kBlock, 0, s>>>(a);
-  }
-}
-
-template <int Q, class S>
-int launch_pair(const lbm::StepArgs& a, cudaStream_t s) {
-  if constexpr (sizeof(S) == 8) {
-    return fail(LBM_ERR_UNSUPPORTED, "paired step has no FP64 form");
-  } else {
-    if constexpr ((Q == 9 || (LBM_QUAD_Q19 && Q == 19)) && sizeof(S) == 2) {
-      if (quad_ok<Q, S>(a)) {
-        if (a.g.n2 % 512 == 0) launch_quad_w<Q, S, 4>(a, s);
-        else if (a.g.n2 % 256 == 0) launch_quad_w<Q, S, 2>(a, s);
-        else launch_quad_w<Q, S, 1>(a, s);
-        return cuda_check(cudaGetLastError(), "k_step_quad launch");
-      }
-    }
-    if constexpr (Q == 9 && sizeof(S) == 2) {
-      if (gquad_ok<Q, S>(a)) {
-        launch_gquad<Q, S>(a, s);
-        return cuda_check(cudaGetLastError(), "k_step_gquad launch");
-      }
-    }
-    if (a.g.n2 % 256 == 0) launch_pair_w<Q, S, 4>(a, s);
-    else if (a.g.n2 % 128 == 0) launch_pair_w<Q, S, 2>(a, s);
-    else if (a.g.n2 % 64 == 0) launch_pair_w<Q, S, 1>(a, s);
-    else launch_gpair<Q, S>(a, s);
-    return cuda_check(cudaGetLastError(), "k_step_pair launch");
-  }
-}
-
-// One state-to-state step (p in -> p out, no moments): paired or one-cell.
-template <int Q, class S>
-int launch_state_step(const lbm_plan* p, const lbm::StepArgs& m, cudaStream_t s) {
-  if (pair_ok<S>(p, m)) return launch_pair<Q, S>(m, s);
-  return launch_step<Q, S>(m, false, s);
-}
-
-template <int Q, class S>
-int launch_step_padded(const lbm::StepArgs& a, cudaStream_t s) {
-  const unsigned grid = grid_for(a.g.ncell);
-  const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
-  const bool force = a.force_mode != 0;
-  if (faces) {
-    if (force) lbm::k_step_padded<Q, S, true, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step_padded<Q, S, true, false><<<grid, lbm::kBlock, 0, s>>>(a);
-  } else {
-    if (force) lbm::k_step_padded<Q, S, false, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step_padded<Q, S, false, false><<<grid, lbm::kBlock, 0, s>>>(a);
-  }
-  return cuda_check(cudaGetLastError(), "k_step_padded launch");
-}
-
-// Collide the whole padded block into the workspace, then the padded step.
-template <int Q, class S>
-int run_padded(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in,
-               void* f_out, char* ws) {
-  (void)p;
-  lbm::StepArgs m = a;
-  m.rho = m.vel = m.prs = nullptr;  // halo moments stay the caller's
-  m.f_in = f_in;
-  m.pout = ws;
-  int rc = launch_prepare<Q, S>(m, s);
-  if (rc) return rc;
-  a.pin = ws;
-  a.f_in = f_in;
-  a.f_out = f_out;
-  return launch_step_padded<Q, S>(a, s);
-}
-
-template <int Q, class S>
-int launch_step_moments_only(const lbm::StepArgs& a, cudaStream_t s) {
-  launch_step_mode<Q, S, lbm::kOutMoments>(a, s);
-  return cuda_check(cudaGetLastError(), "k_step launch");
-}
-
-// One-pass tiled step (lbm_tiled.cuh) for lbm_update and the first step of a
-// rollout: 32-bit IO, rows of a multiple of 4 cells (16-byte copy groups),
-// 16-byte aligned reference-layout buffers that do not overlap, an unpadded
-// whole lattice.
-template <class S>
-bool tiled_ok(const lbm_plan* p, const lbm::StepArgs& a, const void* ws, bool aos_out) {
-  if constexpr (sizeof(typename lbm::StoreT<S>::IO) != 4) {
-    return false;
-  } else {
-    if (p->flags & LBM_PLAN_TWO_PASS) return false;
-    if (p->g.n2 % 4 != 0 || p->g.rstride != p->g.n2 || a.face_inset != 0 || a.force_mode == 3)
-      return false;
-    const uintptr_t fi = reinterpret_cast<uintptr_t>(a.f_in);
-    const uintptr_t fo = reinterpret_cast<uintptr_t>(a.f_out);
-    if (fi % 16 != 0) return false;
-    if (aos_out) {
-      // f_out is written while other blocks still read f_in: no overlap
-      const uintptr_t bytes = static_cast<uintptr_t>(p->g.ncell) * p->Q * 4;
-      if (fo % 16 != 0 || (fo < fi + bytes && fi < fo + bytes)) return false;
-    }
-    return reinterpret_cast<uintptr_t>(ws) % 4 == 0;  // the status word
-  }
-}
-
-// Runs the first step (one-pass tiled kernel, or prepare + a state step),
-// the state steps and the final step; ws holds 1 or 2 state copies (with n > 1
-// also the status word after them).
-template <int Q, class S>
-int run_steps(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in, void* f_out,
-              int64_t n, char* ws) {
-  const size_t sb = align256(state_bytes(p));
-  char* A = ws;
-  char* B = ws + sb;
-  a.f_in = f_in;
-  a.f_out = f_out;
-  int rc;
-  if constexpr (sizeof(typename lbm::StoreT<S>::IO) == 4) {
-    if (n == 1 && tiled_ok<S>(p, a, ws, true)) {
-      // the whole update in one pass; the workspace holds only the status word
-      a.status = reinterpret_cast<int*>(ws);
-      rc = cuda_check(cudaMemsetAsync(a.status, 0, sizeof(int), s), "cudaMemsetAsync");
-      if (rc) return rc;
-      return launch_tiled<Q, S, lbm::kOutAoS>(p, a, s);
-    }
-  }
-  a.pout = A;
-  lbm::StepArgs m = a;  // the first pass and intermediate steps write no moments
-  m.rho = m.vel = m.prs = nullptr;
-  const bool tiled = n > 1 && tiled_ok<S>(p, a, ws + 2 * sb, false);
-  if (tiled) {
-    m.status = reinterpret_cast<int*>(ws + 2 * sb);
-    rc = cuda_check(cudaMemsetAsync(m.status, 0, sizeof(int), s), "cudaMemsetAsync");
-    if (rc) return rc;
-  }
-  if (tiled) {
-    // step 1 straight from the reference layout (p after one step into A)
-    if constexpr (sizeof(typename lbm::StoreT<S>::IO) == 4)
-      rc = launch_tiled<Q, S, lbm::kOutState>(p, m, s);
-    --n;
-  } else {
-    rc = launch_prepare<Q, S>(m, s);
-  }
-  if (rc) return rc;
-  for (int64_t i = 0; i + 1 < n; ++i) {
-    m.pin = A;
-    m.pout = B;
-    rc = launch_state_step<Q, S>(p, m, s);
-    if (rc) return rc;
-    char* t = A;
-    A = B;
-    B = t;
-  }
-  a.pin = A;
-  a.f_out = f_out;
-  return launch_step<Q, S>(a, true, s);
-}
-
-// Rollout that also records the reference state after every `every`-th step
-// (record r = after step (r + 1) every): recorded state steps write f and the
-// moments into the history slots as they collide; the last step's outputs are
-// copied into its slot when it is recorded.
-template <int Q, class S>
-int run_history(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in,
-                void* f_out, int64_t n, int64_t every, const lbm_history* h, char* ws) {
-  const size_t sb = align256(state_bytes(p));
-  const size_t cells = p->g.ncell;
-  const size_t fb = cells * p->Q * p->io, rb = cells * p->io, vb = cells * p->D * p->io;
-  auto slot = [](void* base, size_t bytes, int64_t r) -> void* {
-    return base == nullptr ? nullptr : static_cast<char*>(base) + static_cast<size_t>(r) * bytes;
-  };
-  char* A = ws;
-  char* B = ws + sb;
-  lbm::StepArgs m = a;
-  m.rho = m.vel = m.prs = nullptr;
-  m.f_in = f_in;
-  m.pout = A;
-  int rc = launch_prepare<Q, S>(m, s);
-  if (rc) return rc;
-  for (int64_t i = 1; i < n; ++i) {
-    m.pin = A;
-    m.pout = B;
-    if (i % every == 0) {
-      const int64_t r = i / every - 1;
-      lbm::StepArgs rec = m;
-      rec.f_out = slot(h->f, fb, r);
-      rec.rho = slot(h->density, rb, r);
-      rec.vel = slot(h->velocity, vb, r);
-      rec.prs = slot(h->pressure, rb, r);
-      launch_step_mode<Q, S, lbm::kOutRecord>(rec, s);
-      rc = cuda_check(cudaGetLastError(), "k_step launch");
-    } else {
-      rc = launch_state_step<Q, S>(p, m, s);
-    }
-    if (rc) return rc;
-    char* t = A;
-    A = B;
-    B = t;
-  }
-  const bool last = n % every == 0;
-  const int64_t r = n / every - 1;
-  a.pin = A;
-  a.f_out = f_out;
-  // the last step's moments go to the caller's buffers, or straight to the
-  // history slot when the caller wants none
-  if (last && a.rho == nullptr) a.rho = slot(h->density, rb, r);
-  if (last && a.vel == nullptr) a.vel = slot(h->velocity, vb, r);
-  if (last && a.prs == nullptr) a.prs = slot(h->pressure, rb, r);
-  rc = launch_step<Q, S>(a, true, s);
-  if (rc || !last) return rc;
-  struct { void* dst; const void* src; size_t bytes; } copies[4] = {
-      {slot(h->f, fb, r), f_out, fb},
-      {slot(h->density, rb, r), a.rho, rb},
-      {slot(h->velocity, vb, r), a.vel, vb},
-      {slot(h->pressure, rb, r), a.prs, rb}};
-  for (const auto& c : copies) {
-    if (c.dst == nullptr || c.dst == c.src) continue;
-    rc = cuda_check(cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToDevice, s),
-                    "cudaMemcpyAsync");
-    if (rc) return rc;
-  }
-  return LBM_OK;
-}
-
 template <int Q>
 int dispatch_s(const lbm_plan* p, cudaStream_t s, const lbm::StepArgs& a, const void* f_in,
                void* f_out, int64_t n, char* ws) {
@@ -528,19 +162,10 @@ int do_steps(const lbm_plan* p, lbm_stream_t stream, const void* f_in, void* f_o
                     : dispatch_s<9>(p, s, a, f_in, f_out, n, ws);
 }
 
-constexpr int kReduceBlocks = 148 * 4;
 
 // ---------------------------------------------------------------------------
 // Differentiated rollout: checkpointed forward + reverse sweep
 // ---------------------------------------------------------------------------
-
-struct AdjLayout {
-  int64_t T = 0, K = 0, S = 0;  // steps, checkpoint interval, segments
-  size_t sb = 0;                // bytes of one population copy
-  size_t rho_bytes = 0, slot = 0;
-  size_t A = 0, B = 0, ck = 0, hist = 0, mu0 = 0, mu1 = 0, dF = 0, part = 0, total = 0;
-  bool full = false;  // the moments of every step are kept: no checkpoints, no recompute
-};
 
 int adj_layout(const lbm_plan* p, int64_t T, int64_t K, AdjLayout* L) {
   if (T < 1) return fail(LBM_ERR_INVALID, "n_steps must be >= 1 (got %lld)", (long long)T);
@@ -590,280 +215,9 @@ int adj_check(const lbm_plan* p, const lbm_step_args* args) {
   return LBM_OK;
 }
 
-// Forward pass that keeps (rho^n, u^n) of every step (AdjLayout::full).
-template <int Q, class S>
-int adj_forward_full(cudaStream_t s, lbm::StepArgs a, const void* f_in, void* f_out,
-                     const AdjLayout& L, char* ws) {
-  char* cur = ws + L.A;
-  char* nxt = ws + L.B;
-  lbm::StepArgs m = a;
-  m.prs = nullptr;
-  m.mflags = lbm::kMomRawVelocity;
-  m.f_in = f_in;
-  auto keep = [&](int64_t n) {
-    m.rho = ws + L.hist + static_cast<size_t>(n) * L.slot;
-    m.vel = static_cast<char*>(m.rho) + L.rho_bytes;
-  };
-  keep(0);
-  m.pout = cur;
-  int rc = launch_prepare<Q, S>(m, s);
-  if (rc) return rc;
-  for (int64_t n = 1; n < L.T; ++n) {
-    keep(n);
-    m.pin = cur;
-    m.pout = nxt;
-    rc = launch_step<Q, S>(m, false, s);
-    if (rc) return rc;
-    std::swap(cur, nxt);
-  }
-  // the moments of f^T, raw in walls
-  keep(L.T);
-  m.pin = cur;
-  rc = launch_step_moments_only<Q, S>(m, s);
-  if (rc) return rc;
-  a.pin = cur;
-  a.f_out = f_out;
-  return launch_step<Q, S>(a, true, s);
-}
-
-template <int Q, class S>
-int adj_forward(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in, void* f_out,
-                const AdjLayout& L, char* ws) {
-  if (L.full) return adj_forward_full<Q, S>(s, a, f_in, f_out, L, ws);
-  char* AB[2] = {ws + L.A, ws + L.B};
-  auto slot = [&](int64_t j) { return ws + L.ck + static_cast<size_t>(j - 1) * L.sb; };
-  // Producer of p^m writes into checkpoint j = (m+1)/K when m+1 is a segment start.
-  auto out_for = [&](int64_t m, char* cur) -> char* {
-    if ((m + 1) % L.K == 0 && m + 1 < L.T) return slot((m + 1) / L.K);
-    return cur == AB[0] ? AB[1] : AB[0];
-  };
-  lbm::StepArgs m = a;
-  m.rho = m.vel = m.prs = nullptr;
-  m.f_in = f_in;
-  char* cur = out_for(0, nullptr);
-  m.pout = cur;
-  int rc = launch_prepare<Q, S>(m, s);
-  if (rc) return rc;
-  for (int64_t n = 1; n < L.T; ++n) {
-    char* nxt = out_for(n, cur);
-    m.pin = cur;
-    m.pout = nxt;
-    rc = launch_state_step<Q, S>(p, m, s);
-    if (rc) return rc;
-    cur = nxt;
-  }
-  a.pin = cur;
-  a.f_out = f_out;
-  return launch_step<Q, S>(a, true, s);
-}
-
-template <int Q, class S>
-int adj_backward(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in,
-                 const void* g_rho, const void* g_vel, const void* g_f, double* grad_force,
-                 void* grad_f_in, const AdjLayout& L, char* ws) {
-  using IO = typename lbm::StoreT<S>::IO;
-  char* AB[2] = {ws + L.A, ws + L.B};
-  char* MU[2] = {ws + L.mu0, ws + L.mu1};
-  auto slot = [&](int64_t j) { return ws + L.ck + static_cast<size_t>(j - 1) * L.sb; };
-  auto hist_rho = [&](int64_t j) { return ws + L.hist + static_cast<size_t>(j) * L.slot; };
-  auto hist_vel = [&](int64_t j) { return hist_rho(j) + L.rho_bytes; };
-  double* dF = reinterpret_cast<double*>(ws + L.dF);
-  const unsigned grid = grid_for(p->g.ncell);
-
-  lbm::AdjArgs q{};
-  q.g = p->g;
-  q.omega = a.omega;
-  q.guo_c = a.guo_c;
-  q.force_mode = a.force_mode;
-  for (int d = 0; d < 3; ++d) q.force[d] = a.force[d];
-  q.force_field = a.force_field;
-  q.wall = a.wall;
-  q.dF = grad_force != nullptr ? dF : nullptr;
-  const bool force = a.force_mode != 0;
-
-  lbm::StepArgs m = a;  // recompute steps: moments into the history, raw velocity
-  m.prs = nullptr;
-  m.mflags = lbm::kMomRawVelocity;
-  m.f_in = f_in;
-  int mu = 0;  // MU[mu] holds mu^{n+1}
-  int rc = LBM_OK;
-  const int64_t segments = L.full ? 1 : L.S;
-  for (int64_t sg = segments - 1; sg >= 0; --sg) {
-    const int64_t n0 = sg * L.K;
-    const int64_t n1 = L.full || n0 + L.K > L.T ? L.T : n0 + L.K;
-    if (!L.full) {
-      // (rho^n, u^n) for n in [n0, n1): recompute from the segment's checkpoint
-      char* cur = AB[0];
-      m.rho = hist_rho(0);
-      m.vel = hist_vel(0);
-      m.pout = cur;
-      if (sg == 0) {
-        rc = launch_prepare<Q, S>(m, s);
-      } else {
-        m.pin = slot(sg);
-        rc = launch_step<Q, S>(m, false, s);
-      }
-      if (rc) return rc;
-      for (int64_t n = n0 + 1; n < n1; ++n) {
-        char* nxt = cur == AB[0] ? AB[1] : AB[0];
-        m.rho = hist_rho(n - n0);
-        m.vel = hist_vel(n - n0);
-        m.pin = cur;
-        m.pout = nxt;
-        rc = launch_step<Q, S>(m, false, s);
-        if (rc) return rc;
-        cur = nxt;
-      }
-      if (sg == L.S - 1) {  // moments of f^T
-        m.rho = hist_rho(n1 - n0);
-        m.vel = hist_vel(n1 - n0);
-        m.pin = cur;
-        rc = launch_step_moments_only<Q, S>(m, s);
-        if (rc) return rc;
-      }
-    }
-    if (sg == segments - 1) {
-      // lambda^T from the output gradients
-      q.rho = hist_rho(n1 - n0);
-      q.vel = hist_vel(n1 - n0);
-      q.g_rho = g_rho;
-      q.g_vel = g_vel;
-      q.g_f = g_f;
-      q.mout = MU[mu];
-      lbm::k_adj_init<Q, S><<<grid, lbm::kBlock, 0, s>>>(q);
-      rc = cuda_check(cudaGetLastError(), "k_adj_init launch");
-      if (rc) return rc;
-    }
-    for (int64_t n = n1 - 1; n >= n0; --n) {
-      q.rho = hist_rho(n - n0);
-      q.vel = hist_vel(n - n0);
-      q.min = MU[mu];
-      q.mout = MU[1 - mu];
-      const bool aos = n == 0 && grad_f_in != nullptr;
-      q.grad_f0 = grad_f_in;
-      if (aos) {
-        if (force) lbm::k_adj_step<Q, S, true, lbm::kAdjOutAoS><<<grid, lbm::kBlock, 0, s>>>(q);
-        else lbm::k_adj_step<Q, S, false, lbm::kAdjOutAoS><<<grid, lbm::kBlock, 0, s>>>(q);
-      } else {
-        if (force) lbm::k_adj_step<Q, S, true, lbm::kAdjOutState><<<grid, lbm::kBlock, 0, s>>>(q);
-        else lbm::k_adj_step<Q, S, false, lbm::kAdjOutState><<<grid, lbm::kBlock, 0, s>>>(q);
-      }
-      rc = cuda_check(cudaGetLastError(), "k_adj_step launch");
-      if (rc) return rc;
-      mu = 1 - mu;
-    }
-  }
-  if (grad_force != nullptr) {
-    if (a.force_mode == LBM_FORCE_UNIFORM) {
-      double* part = reinterpret_cast<double*>(ws + L.part);
-      if (p->D == 3)
-        lbm::k_field_sum_part<3><<<kReduceBlocks, lbm::kReduceThreads, 0, s>>>(dF, p->g.ncell, part);
-      else
-        lbm::k_field_sum_part<2><<<kReduceBlocks, lbm::kReduceThreads, 0, s>>>(dF, p->g.ncell, part);
-      lbm::k_field_sum_final<<<1, lbm::kReduceThreads, 0, s>>>(part, kReduceBlocks, p->D,
-                                                              grad_force);
-      rc = cuda_check(cudaGetLastError(), "k_field_sum launch");
-    } else {
-      rc = cuda_check(cudaMemcpyAsync(grad_force, dF,
-                                      static_cast<size_t>(p->g.ncell) * p->D * sizeof(double),
-                                      cudaMemcpyDeviceToDevice, s),
-                      "cudaMemcpyAsync");
-    }
-  }
-  (void)sizeof(IO);
-  return rc;
-}
-
 // ---------------------------------------------------------------------------
 // Batched ensemble (host side)
 // ---------------------------------------------------------------------------
-
-// A contiguous range [t0, t1) of the tile list whose instances are stepped
-// together; grid = blocks of the persistent launch for that range; pair = its
-// state steps run the paired kernel (16-bit storage, even rows).
-struct TileRange {
-  uint32_t t0, t1;  // reference-layout tiles (prepare, one-cell steps, last step)
-  uint32_t s0, s1;  // state-layout tiles (paired state steps)
-  unsigned grid, sgrid;
-  bool pair;        // state steps paired
-  bool pad;         // ... with padded state rows
-};
-
-// Prepare pass over all tiles, then for each instance group its n - 1 state
-// steps and its last step.  A group whose two population copies fit in L2
-// stays there for all of its steps.
-template <int Q, class S, int MODE, int SPEC>
-void batched_launch(bool pair, bool pad, const lbm::StepArgs* args, const lbm::BatchTile* t,
-                    uint32_t nt, unsigned grid, int which, cudaStream_t s) {
-  if constexpr (MODE == lbm::kOutState && sizeof(S) == 2) {
-    if (pair) {
-      if (pad) lbm::k_batched_pair<Q, S, SPEC, true><<<grid, lbm::kBlock, 0, s>>>(args, t, nt, which);
-      else lbm::k_batched_pair<Q, S, SPEC, false><<<grid, lbm::kBlock, 0, s>>>(args, t, nt, which);
-      return;
-    }
-  }
-  lbm::k_batched_step<Q, S, MODE, SPEC><<<grid, lbm::kBlock, 0, s>>>(args, t, nt, which);
-}
-
-// spec: 0 = per-tile run-time choice, else 1 + 2 FACES + FORCE shared by all members
-template <int Q, class S, int MODE>
-void batched_step(int spec, bool pair, bool pad, const lbm::StepArgs* args,
-                  const lbm::BatchTile* t, uint32_t nt, unsigned grid, int which, cudaStream_t s) {
-  switch (spec) {
-    case 1: batched_launch<Q, S, MODE, 1>(pair, pad, args, t, nt, grid, which, s); break;
-    case 2: batched_launch<Q, S, MODE, 2>(pair, pad, args, t, nt, grid, which, s); break;
-    case 3: batched_launch<Q, S, MODE, 3>(pair, pad, args, t, nt, grid, which, s); break;
-    case 4: batched_launch<Q, S, MODE, 4>(pair, pad, args, t, nt, grid, which, s); break;
-    default: batched_launch<Q, S, MODE, 0>(pair, pad, args, t, nt, grid, which, s); break;
-  }
-}
-
-template <int Q, class S>
-int batched_run(const lbm::StepArgs* args, const lbm::BatchTile* tiles,
-                const lbm::BatchTile* stiles, uint32_t ntiles, unsigned grid_all,
-                const std::vector<TileRange>& groups, int64_t n, cudaStream_t s,
-                cudaStream_t side, bool use_graph, int spec) {
-  lbm::k_batched_prepare<Q, S><<<grid_all, lbm::kBlock, 0, s>>>(args, tiles, ntiles);
-  int rc = cuda_check(cudaGetLastError(), "k_batched_prepare launch");
-  if (rc) return rc;
-  cudaStream_t ls = s;
-  cudaGraph_t graph = nullptr;
-  if (use_graph) {
-    // The step sequence is recorded on the batch's own stream (capture only
-    // records, nothing runs there) and replayed on the caller's stream, after
-    // the work already queued on it.
-    rc = cuda_check(cudaStreamBeginCapture(side, cudaStreamCaptureModeThreadLocal),
-                    "cudaStreamBeginCapture");
-    if (rc) return rc;
-    ls = side;
-  }
-  for (const TileRange& r : groups) {
-    const lbm::BatchTile* t = tiles + r.t0;
-    const uint32_t nt = r.t1 - r.t0;
-    for (int64_t k = 1; k < n; ++k) {
-      if (r.pair)
-        batched_step<Q, S, lbm::kOutState>(spec, true, r.pad, args, stiles + r.s0, r.s1 - r.s0,
-                                           r.sgrid, static_cast<int>(k % 2), ls);
-      else
-        batched_step<Q, S, lbm::kOutState>(spec, false, false, args, t, nt, r.grid,
-                                           static_cast<int>(k % 2), ls);
-    }
-    batched_step<Q, S, lbm::kOutAoS>(spec, false, false, args, t, nt, r.grid, 2, ls);
-  }
-  rc = cuda_check(cudaGetLastError(), "k_batched_step launch");
-  if (use_graph) {
-    const int rc2 = cuda_check(cudaStreamEndCapture(side, &graph), "cudaStreamEndCapture");
-    if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
-    if (rc2) return rc2;
-    cudaGraphExec_t exec = nullptr;
-    rc = cuda_check(cudaGraphInstantiate(&exec, graph, 0), "cudaGraphInstantiate");
-    cudaGraphDestroy(graph);
-    if (rc) return rc;
-    rc = cuda_check(cudaGraphLaunch(exec, s), "cudaGraphLaunch");
-    cudaGraphExecDestroy(exec);  // released once the launched graph completes
-  }
-  return rc;
-}
 
 }  // namespace
 
@@ -1091,18 +445,6 @@ int lbm_rollout_history(const lbm_plan* p, lbm_stream_t stream, const void* f_in
 
 namespace {
 
-enum StateOp { kFromF, kStep, kToF };
-
-template <int Q, class S>
-int state_op(StateOp op, const lbm::StepArgs& a, cudaStream_t s) {
-  if (op == kFromF) return launch_prepare<Q, S>(a, s);
-  if (op == kStep) {
-    launch_step_mode<Q, S, lbm::kOutState>(a, s);  // one cell per thread, any storage
-    return cuda_check(cudaGetLastError(), "k_step launch");
-  }
-  return launch_step<Q, S>(a, true, s);
-}
-
 template <int Q>
 int state_op_s(const lbm_plan* p, StateOp op, const lbm::StepArgs& a, cudaStream_t s) {
   switch (p->storage) {
@@ -1186,118 +528,6 @@ namespace {
 size_t pipe_workspace(const lbm_plan* p) {
   const size_t n = p->g.ncell;
   return 2 * align256(state_bytes(p)) + 2 * align256(7 * n * p->io) + align256(3 * n * p->io);
-}
-
-// Single-phase pipe rollout: one fused launch per step (k_pipe_step: D3Q19
-// pull step + the tracer of the same cell), tracer populations ping-ponged
-// between two plane sets.
-template <class S>
-int run_pipe(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in, void* f_out,
-             const void* t_in, void* t_out, int64_t n, double tau_tracer, void* tracer_out,
-             char* ws) {
-  using IO = typename lbm::StoreT<S>::IO;
-  const size_t cells = p->g.ncell;
-  const size_t sb = align256(state_bytes(p)), tb = align256(7 * cells * p->io);
-  char* A = ws;
-  char* B = ws + sb;
-  char* T[2] = {ws + 2 * sb, ws + 2 * sb + tb};
-  const unsigned grid = grid_for(p->g.ncell);
-  lbm::TracerArgs t{};
-  t.g = p->g;
-  t.wall = a.wall;
-  t.inv_tau = 1.0 / tau_tracer;
-  t.f7_in = t_in;
-  t.tout = T[0];
-  lbm::k_tracer_prepare<IO><<<grid, lbm::kBlock, 0, s>>>(t);
-  int rc = cuda_check(cudaGetLastError(), "k_tracer_prepare launch");
-  if (rc) return rc;
-  lbm::StepArgs m = a;
-  m.rho = m.prs = m.vel = nullptr;
-  m.f_in = f_in;
-  m.pout = A;
-  rc = launch_prepare<19, S>(m, s);
-  if (rc) return rc;
-  int cur = 0;
-  for (int64_t i = 1; i < n; ++i) {
-    m.pin = A;
-    m.pout = B;
-    t.tin = T[cur];
-    t.tout = T[1 - cur];
-    lbm::k_pipe_step<S, false><<<grid, lbm::kBlock, 0, s>>>(m, t);
-    rc = cuda_check(cudaGetLastError(), "k_pipe_step launch");
-    if (rc) return rc;
-    cur = 1 - cur;
-    std::swap(A, B);
-  }
-  a.pin = A;
-  a.f_out = f_out;
-  a.prs = nullptr;
-  a.mflags &= ~lbm::kMomRawVelocity;
-  t.tin = T[cur];
-  t.tout = T[1 - cur];
-  lbm::k_pipe_step<S, true><<<grid, lbm::kBlock, 0, s>>>(a, t);
-  rc = cuda_check(cudaGetLastError(), "k_pipe_step launch");
-  if (rc) return rc;
-  cur = 1 - cur;
-  t.tin = T[cur];
-  t.f7_out = t_out;
-  t.tracer_out = tracer_out;
-  lbm::k_tracer_final<IO><<<grid, lbm::kBlock, 0, s>>>(t);
-  return cuda_check(cudaGetLastError(), "k_tracer_final launch");
-}
-
-// Multiphase pipe step (G != 0): two passes per step over pre-collision
-// population planes (lbm_multiphase.cuh); the workspace holds two population
-// sets and the psi plane, inside the single-phase layout.
-template <class R>
-int run_pipe_mp(const lbm_plan* p, cudaStream_t s, const lbm::StepArgs& a,
-                const lbm_pipe_args* pa, const void* f_in, void* f_out, const void* t_in,
-                void* t_out, int64_t n, const lbm_moments* out, void* tracer_out, char* ws) {
-  const size_t cells = p->g.ncell;
-  const size_t sb = align256(state_bytes(p));
-  char* A = ws;
-  char* B = ws + sb;
-  lbm::MPArgs m{};
-  m.s = a;
-  m.G = pa->G;
-  m.rho0 = pa->rho_0;
-  m.psi_wall = pa->rho_0 * (1.0 - std::exp(-pa->rho_wall / pa->rho_0));
-  m.rho_gas = pa->rho_gas;
-  m.drho = pa->rho_liquid - pa->rho_gas;
-  m.psi = ws + 2 * sb;
-  m.f_aos_in = f_in;
-  const unsigned grid = grid_for(p->g.ncell);
-  // step 1: psi of the reference f, then its collide into A
-  lbm::k_mp_density<R, lbm::kMPFirst><<<grid, lbm::kBlock, 0, s>>>(m);
-  int rc = cuda_check(cudaGetLastError(), "k_mp_density launch");
-  if (rc) return rc;
-  m.fout = A;
-  lbm::k_mp_collide<R, true><<<grid, lbm::kBlock, 0, s>>>(m);
-  rc = cuda_check(cudaGetLastError(), "k_mp_collide launch");
-  if (rc) return rc;
-  // steps 2..n: both passes pull from the post-collision planes
-  for (int64_t i = 1; i < n; ++i) {
-    m.fin = A;
-    m.fout = B;
-    lbm::k_mp_density<R, lbm::kMPStep><<<grid, lbm::kBlock, 0, s>>>(m);
-    rc = cuda_check(cudaGetLastError(), "k_mp_density launch");
-    if (rc) return rc;
-    lbm::k_mp_collide<R, false><<<grid, lbm::kBlock, 0, s>>>(m);
-    rc = cuda_check(cudaGetLastError(), "k_mp_collide launch");
-    if (rc) return rc;
-    std::swap(A, B);
-  }
-  m.fin = A;
-  m.f_aos_out = f_out;
-  m.rho_out = out != nullptr ? out->density : nullptr;
-  m.vel_out = out != nullptr ? out->velocity : nullptr;
-  m.tracer_out = tracer_out;
-  lbm::k_mp_density<R, lbm::kMPLast><<<grid, lbm::kBlock, 0, s>>>(m);
-  rc = cuda_check(cudaGetLastError(), "k_mp_density launch");
-  if (rc) return rc;
-  // tracer_f is not evolved in multiphase mode (lbm_pipe.py:858-860)
-  return cuda_check(cudaMemcpyAsync(t_out, t_in, 7 * cells * sizeof(R), cudaMemcpyDeviceToDevice, s),
-                    "tracer_f copy");
 }
 
 }  // namespace

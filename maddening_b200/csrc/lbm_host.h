@@ -7,7 +7,9 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstdint>
+#include <vector>
 
 #include "../../include/lbm_b200.h"
 #include "lbm_kernels.cuh"
@@ -26,6 +28,85 @@ struct lbm_plan {
 int fail(int code, const char* fmt, ...);
 // LBM_OK, or fail(LBM_ERR_CUDA, "<what>: <CUDA message>").
 int cuda_check(cudaError_t e, const char* what);
+
+inline size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
+
+inline size_t state_bytes(const lbm_plan* p) {
+  return static_cast<size_t>(p->Q) * static_cast<size_t>(p->g.ncell) * p->elem;
+}
+
+inline unsigned grid_for(uint64_t n) { return static_cast<unsigned>((n + lbm::kBlock - 1) / lbm::kBlock); }
+
+// ---- Launchers, one unit per lattice and storage (lbm_steps.cu) ----------
+// p = C(f) of the reference state a.f_in into a.pout.
+template <int Q, class S>
+int launch_prepare(const lbm::StepArgs& a, cudaStream_t s);
+// One step, one cell per thread: the next state, or (final_aos) f_bc and moments.
+template <int Q, class S>
+int launch_step(const lbm::StepArgs& a, bool final_aos, cudaStream_t s);
+template <int Q, class S>
+int launch_step_moments_only(const lbm::StepArgs& a, cudaStream_t s);
+template <int Q, class S>
+int run_padded(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in, void* f_out,
+               char* ws);
+template <int Q, class S>
+int run_steps(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in, void* f_out,
+              int64_t n, char* ws);
+template <int Q, class S>
+int run_history(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in,
+                void* f_out, int64_t n, int64_t every, const lbm_history* h, char* ws);
+enum StateOp { kFromF, kStep, kToF };
+template <int Q, class S>
+int state_op(StateOp op, const lbm::StepArgs& a, cudaStream_t s);
+// One state-to-state step in the form the plan and the storage take.
+template <int Q, class S>
+int launch_state_step(const lbm_plan* p, const lbm::StepArgs& m, cudaStream_t s);
+
+// ---- Differentiated rollout (lbm_grad.cu) -----------------------------------
+constexpr int kReduceBlocks = 148 * 4;
+struct AdjLayout {
+  int64_t T = 0, K = 0, S = 0;  // steps, checkpoint interval, segments
+  size_t sb = 0;                // bytes of one population copy
+  size_t rho_bytes = 0, slot = 0;
+  size_t A = 0, B = 0, ck = 0, hist = 0, mu0 = 0, mu1 = 0, dF = 0, part = 0, total = 0;
+  bool full = false;  // the moments of every step are kept: no checkpoints, no recompute
+};
+
+template <int Q, class S>
+int adj_forward(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in, void* f_out,
+                const AdjLayout& L, char* ws);
+template <int Q, class S>
+int adj_backward(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in,
+                 const void* g_rho, const void* g_vel, const void* g_f, double* grad_force,
+                 void* grad_f_in, const AdjLayout& L, char* ws);
+
+// ---- Batched ensemble (lbm_batch.cu) ----------------------------------------
+// A contiguous range [t0, t1) of the tile list whose instances are stepped
+// together; grid = blocks of the persistent launch for that range; pair = its
+// state steps run the paired kernel (16-bit storage, even rows).
+struct TileRange {
+  uint32_t t0, t1;  // reference-layout tiles (prepare, one-cell steps, last step)
+  uint32_t s0, s1;  // state-layout tiles (paired state steps)
+  unsigned grid, sgrid;
+  bool pair;        // state steps paired
+  bool pad;         // ... with padded state rows
+};
+
+template <int Q, class S>
+int batched_run(const lbm::StepArgs* args, const lbm::BatchTile* tiles,
+                const lbm::BatchTile* stiles, uint32_t ntiles, unsigned grid_all,
+                const std::vector<TileRange>& groups, int64_t n, cudaStream_t s,
+                cudaStream_t side, bool use_graph, int spec);
+
+// ---- Pipe node (lbm_pipe.cu) -------------------------------------------------
+template <class S>
+int run_pipe(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in, void* f_out,
+             const void* t_in, void* t_out, int64_t n, double tau_tracer, void* tracer_out,
+             char* ws);
+template <class R>
+int run_pipe_mp(const lbm_plan* p, cudaStream_t s, const lbm::StepArgs& a,
+                const lbm_pipe_args* pa, const void* f_in, void* f_out, const void* t_in,
+                void* t_out, int64_t n, const lbm_moments* out, void* tracer_out, char* ws);
 
 // One-pass tiled step (lbm_tiled.cuh, launched from lbm_tiled.cu) for 32-bit
 // IO: MODE lbm::kOutAoS (a whole update) or lbm::kOutState (the first step of a

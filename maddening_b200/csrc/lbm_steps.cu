@@ -1,0 +1,389 @@
+// Launches and rollouts of the step kernels for one lattice and storage: the
+// build compiles this file once per pair (LBM_UNIT_Q, LBM_UNIT_S), so that the
+// units are compiled in parallel and each as a whole.
+#include <cuda_runtime.h>
+
+#include "lbm_host.h"
+#include "lbm_kernels.cuh"
+#include "lbm_pair.cuh"
+
+namespace {
+
+template <int Q, class S, int MODE>
+void launch_step_mode(const lbm::StepArgs& a, cudaStream_t s) {
+  const unsigned grid = grid_for(a.cell_end - a.cell0);
+  const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
+  const bool force = a.force_mode != 0;
+  if (faces) {
+    if (force) lbm::k_step<Q, S, MODE, true, true><<<grid, lbm::kBlock, 0, s>>>(a);
+    else lbm::k_step<Q, S, MODE, true, false><<<grid, lbm::kBlock, 0, s>>>(a);
+  } else {
+    if (force) lbm::k_step<Q, S, MODE, false, true><<<grid, lbm::kBlock, 0, s>>>(a);
+    else lbm::k_step<Q, S, MODE, false, false><<<grid, lbm::kBlock, 0, s>>>(a);
+  }
+}
+
+// Paired-cell state step (lbm_pair.cuh): the default for 16-bit storage,
+// opt-in for FP32 (LBM_PLAN_PAIRED_CELLS), off with LBM_PLAN_SINGLE_CELLS.
+// Rows of even length (row segments when they split into warps of 64 cells,
+// instance-wide pairs otherwise); state planes and the wall mask aligned for
+// the pair width.
+template <class S>
+bool pair_ok(const lbm_plan* p, const lbm::StepArgs& a) {
+  if constexpr (sizeof(S) == 8) {
+    return false;
+  } else {
+    if (p->flags & LBM_PLAN_SINGLE_CELLS) return false;
+    if (sizeof(S) == 4 && !(p->flags & LBM_PLAN_PAIRED_CELLS)) return false;
+    const uintptr_t al = 2 * sizeof(S);
+    return p->g.n2 % 2 == 0 && reinterpret_cast<uintptr_t>(a.pin) % al == 0 &&
+           reinterpret_cast<uintptr_t>(a.pout) % al == 0 &&
+           reinterpret_cast<uintptr_t>(a.wall) % 2 == 0;
+  }
+}
+
+template <int Q, class S, int W>
+void launch_pair_w(const lbm::StepArgs& a, cudaStream_t s) {
+  const dim3 grid(a.g.n0 * a.g.n1, a.g.n2 / (64 * W));
+  const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
+  const bool force = a.force_mode != 0;
+  if (faces) {
+    if (force) lbm::k_step_pair<Q, S, true, true, W><<<grid, 32 * W, 0, s>>>(a);
+    else lbm::k_step_pair<Q, S, true, false, W><<<grid, 32 * W, 0, s>>>(a);
+  } else {
+    if (force) lbm::k_step_pair<Q, S, false, true, W><<<grid, 32 * W, 0, s>>>(a);
+    else lbm::k_step_pair<Q, S, false, false, W><<<grid, 32 * W, 0, s>>>(a);
+  }
+}
+
+template <int Q, class S, int W>
+void launch_quad_w(const lbm::StepArgs& a, cudaStream_t s) {
+  const dim3 grid(a.g.n0 * a.g.n1, a.g.n2 / (128 * W));
+  const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
+  const bool force = a.force_mode != 0;
+  if (faces) {
+    if (force) lbm::k_step_quad<Q, S, true, true, W><<<grid, 32 * W, 0, s>>>(a);
+    else lbm::k_step_quad<Q, S, true, false, W><<<grid, 32 * W, 0, s>>>(a);
+  } else {
+    if (force) lbm::k_step_quad<Q, S, false, true, W><<<grid, 32 * W, 0, s>>>(a);
+    else lbm::k_step_quad<Q, S, false, false, W><<<grid, 32 * W, 0, s>>>(a);
+  }
+}
+
+// The four-cell form (16-bit storage): rows of a multiple of 128 cells,
+// unpadded state rows, 8-byte aligned planes and a 4-byte aligned wall mask.
+// D3Q19 also takes it (a B200 sweep at 256^3: 79.2k MLUPS FP16 against 71.7k
+// for pairs, at 20 resident warps and 96 registers) on rows of a multiple of
+// 256 cells: with one-warp blocks (rows of 128) it keeps 15 warps resident and
+// loses to pairs.
+#ifndef LBM_QUAD_Q19
+#define LBM_QUAD_Q19 1
+#endif
+template <int Q, class S>
+bool quad_ok(const lbm::StepArgs& a) {
+  return (Q == 9 || (LBM_QUAD_Q19 && Q == 19)) && sizeof(S) == 2 &&
+         a.g.n2 % (Q == 19 ? 256 : 128) == 0 && a.g.rstride == a.g.n2 &&
+         a.g.pstride % 4 == 0 && reinterpret_cast<uintptr_t>(a.pin) % 8 == 0 &&
+         reinterpret_cast<uintptr_t>(a.pout) % 8 == 0 &&
+         reinterpret_cast<uintptr_t>(a.wall) % 4 == 0;
+}
+
+template <int Q, class S>
+void launch_gquad(const lbm::StepArgs& a, cudaStream_t s) {
+  const unsigned grid = grid_for(a.g.ncell / 4);
+  const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
+  const bool force = a.force_mode != 0;
+  if (faces) {
+    if (force) lbm::k_step_gquad<Q, S, true, true><<<grid, lbm::kBlock, 0, s>>>(a);
+    else lbm::k_step_gquad<Q, S, true, false><<<grid, lbm::kBlock, 0, s>>>(a);
+  } else {
+    if (force) lbm::k_step_gquad<Q, S, false, true><<<grid, lbm::kBlock, 0, s>>>(a);
+    else lbm::k_step_gquad<Q, S, false, false><<<grid, lbm::kBlock, 0, s>>>(a);
+  }
+}
+
+// The instance-wide four-cell form: D2Q9 with 16-bit storage, rows of a
+// multiple of 4 cells (a quad never spans two rows), the same alignment as the
+// row form (4000^2 channel: 148.9k MLUPS against 114.4k for pairs).  D3Q19
+// keeps pairs there: with per-lane rows its 96-register budget spills and it
+// lost (48.3k against 61.9k at 160^3; 56.4k at 128 registers and 16 warps).
+template <int Q, class S>
+bool gquad_ok(const lbm::StepArgs& a) {
+  return Q == 9 && sizeof(S) == 2 && a.g.n2 % 4 == 0 &&
+         a.g.rstride == a.g.n2 && a.g.pstride % 4 == 0 &&
+         reinterpret_cast<uintptr_t>(a.pin) % 8 == 0 &&
+         reinterpret_cast<uintptr_t>(a.pout) % 8 == 0 &&
+         reinterpret_cast<uintptr_t>(a.wall) % 4 == 0;
+}
+
+template <int Q, class S>
+void launch_gpair(const lbm::StepArgs& a, cudaStream_t s) {
+  const unsigned grid = grid_for(a.g.ncell / 2);
+  const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
+  const bool force = a.force_mode != 0;
+  if (faces) {
+    if (force) lbm::k_step_gpair<Q, S, true, true><<<grid, lbm::kBlock, 0, s>>>(a);
+    else lbm::k_step_gpair<Q, S, true, false><<<grid, lbm::kBlock, 0, s>>>(a);
+  } else {
+    if (force) lbm::k_step_gpair<Q, S, false, true><<<grid, lbm::kBlock, 0, s>>>(a);
+    else lbm::k_step_gpair<Q, S, false, false><<<grid, lbm::kBlock, 0, s>>>(a);
+  }
+}
+
+template <int Q, class S>
+int launch_pair(const lbm::StepArgs& a, cudaStream_t s) {
+  if constexpr (sizeof(S) == 8) {
+    return fail(LBM_ERR_UNSUPPORTED, "paired step has no FP64 form");
+  } else {
+    if constexpr ((Q == 9 || (LBM_QUAD_Q19 && Q == 19)) && sizeof(S) == 2) {
+      if (quad_ok<Q, S>(a)) {
+        if (a.g.n2 % 512 == 0) launch_quad_w<Q, S, 4>(a, s);
+        else if (a.g.n2 % 256 == 0) launch_quad_w<Q, S, 2>(a, s);
+        else launch_quad_w<Q, S, 1>(a, s);
+        return cuda_check(cudaGetLastError(), "k_step_quad launch");
+      }
+    }
+    if constexpr (Q == 9 && sizeof(S) == 2) {
+      if (gquad_ok<Q, S>(a)) {
+        launch_gquad<Q, S>(a, s);
+        return cuda_check(cudaGetLastError(), "k_step_gquad launch");
+      }
+    }
+    if (a.g.n2 % 256 == 0) launch_pair_w<Q, S, 4>(a, s);
+    else if (a.g.n2 % 128 == 0) launch_pair_w<Q, S, 2>(a, s);
+    else if (a.g.n2 % 64 == 0) launch_pair_w<Q, S, 1>(a, s);
+    else launch_gpair<Q, S>(a, s);
+    return cuda_check(cudaGetLastError(), "k_step_pair launch");
+  }
+}
+
+template <int Q, class S>
+int launch_step_padded(const lbm::StepArgs& a, cudaStream_t s) {
+  const unsigned grid = grid_for(a.g.ncell);
+  const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
+  const bool force = a.force_mode != 0;
+  if (faces) {
+    if (force) lbm::k_step_padded<Q, S, true, true><<<grid, lbm::kBlock, 0, s>>>(a);
+    else lbm::k_step_padded<Q, S, true, false><<<grid, lbm::kBlock, 0, s>>>(a);
+  } else {
+    if (force) lbm::k_step_padded<Q, S, false, true><<<grid, lbm::kBlock, 0, s>>>(a);
+    else lbm::k_step_padded<Q, S, false, false><<<grid, lbm::kBlock, 0, s>>>(a);
+  }
+  return cuda_check(cudaGetLastError(), "k_step_padded launch");
+}
+
+// One-pass tiled step (lbm_tiled.cuh) for lbm_update and the first step of a
+// rollout: 32-bit IO, rows of a multiple of 4 cells (16-byte copy groups),
+// 16-byte aligned reference-layout buffers that do not overlap, an unpadded
+// whole lattice.
+template <class S>
+bool tiled_ok(const lbm_plan* p, const lbm::StepArgs& a, const void* ws, bool aos_out) {
+  if constexpr (sizeof(typename lbm::StoreT<S>::IO) != 4) {
+    return false;
+  } else {
+    if (p->flags & LBM_PLAN_TWO_PASS) return false;
+    if (p->g.n2 % 4 != 0 || p->g.rstride != p->g.n2 || a.face_inset != 0 || a.force_mode == 3)
+      return false;
+    const uintptr_t fi = reinterpret_cast<uintptr_t>(a.f_in);
+    const uintptr_t fo = reinterpret_cast<uintptr_t>(a.f_out);
+    if (fi % 16 != 0) return false;
+    if (aos_out) {
+      // f_out is written while other blocks still read f_in: no overlap
+      const uintptr_t bytes = static_cast<uintptr_t>(p->g.ncell) * p->Q * 4;
+      if (fo % 16 != 0 || (fo < fi + bytes && fi < fo + bytes)) return false;
+    }
+    return reinterpret_cast<uintptr_t>(ws) % 4 == 0;  // the status word
+  }
+}
+
+}  // namespace
+
+template <int Q, class S>
+int launch_prepare(const lbm::StepArgs& a, cudaStream_t s) {
+  const unsigned grid = grid_for(a.g.ncell);
+  if (a.force_mode != 0)
+    lbm::k_prepare<Q, S, true><<<grid, lbm::kBlock, 0, s>>>(a);
+  else
+    lbm::k_prepare<Q, S, false><<<grid, lbm::kBlock, 0, s>>>(a);
+  return cuda_check(cudaGetLastError(), "k_prepare launch");
+}
+
+template <int Q, class S>
+int launch_step(const lbm::StepArgs& a, bool final_aos, cudaStream_t s) {
+  if (final_aos) launch_step_mode<Q, S, lbm::kOutAoS>(a, s);
+  else launch_step_mode<Q, S, lbm::kOutState>(a, s);
+  return cuda_check(cudaGetLastError(), "k_step launch");
+}
+
+template <int Q, class S>
+int launch_step_moments_only(const lbm::StepArgs& a, cudaStream_t s) {
+  launch_step_mode<Q, S, lbm::kOutMoments>(a, s);
+  return cuda_check(cudaGetLastError(), "k_step launch");
+}
+
+// One state-to-state step (p in -> p out, no moments): paired or one-cell.
+template <int Q, class S>
+int launch_state_step(const lbm_plan* p, const lbm::StepArgs& m, cudaStream_t s) {
+  if (pair_ok<S>(p, m)) return launch_pair<Q, S>(m, s);
+  return launch_step<Q, S>(m, false, s);
+}
+
+// Collide the whole padded block into the workspace, then the padded step.
+template <int Q, class S>
+int run_padded(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in,
+               void* f_out, char* ws) {
+  (void)p;
+  lbm::StepArgs m = a;
+  m.rho = m.vel = m.prs = nullptr;  // halo moments stay the caller's
+  m.f_in = f_in;
+  m.pout = ws;
+  int rc = launch_prepare<Q, S>(m, s);
+  if (rc) return rc;
+  a.pin = ws;
+  a.f_in = f_in;
+  a.f_out = f_out;
+  return launch_step_padded<Q, S>(a, s);
+}
+
+// Runs the first step (one-pass tiled kernel, or prepare + a state step),
+// the state steps and the final step; ws holds 1 or 2 state copies (with n > 1
+// also the status word after them).
+template <int Q, class S>
+int run_steps(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in, void* f_out,
+              int64_t n, char* ws) {
+  const size_t sb = align256(state_bytes(p));
+  char* A = ws;
+  char* B = ws + sb;
+  a.f_in = f_in;
+  a.f_out = f_out;
+  int rc;
+  if constexpr (sizeof(typename lbm::StoreT<S>::IO) == 4) {
+    if (n == 1 && tiled_ok<S>(p, a, ws, true)) {
+      // the whole update in one pass; the workspace holds only the status word
+      a.status = reinterpret_cast<int*>(ws);
+      rc = cuda_check(cudaMemsetAsync(a.status, 0, sizeof(int), s), "cudaMemsetAsync");
+      if (rc) return rc;
+      return launch_tiled<Q, S, lbm::kOutAoS>(p, a, s);
+    }
+  }
+  a.pout = A;
+  lbm::StepArgs m = a;  // the first pass and intermediate steps write no moments
+  m.rho = m.vel = m.prs = nullptr;
+  const bool tiled = n > 1 && tiled_ok<S>(p, a, ws + 2 * sb, false);
+  if (tiled) {
+    m.status = reinterpret_cast<int*>(ws + 2 * sb);
+    rc = cuda_check(cudaMemsetAsync(m.status, 0, sizeof(int), s), "cudaMemsetAsync");
+    if (rc) return rc;
+  }
+  if (tiled) {
+    // step 1 straight from the reference layout (p after one step into A)
+    if constexpr (sizeof(typename lbm::StoreT<S>::IO) == 4)
+      rc = launch_tiled<Q, S, lbm::kOutState>(p, m, s);
+    --n;
+  } else {
+    rc = launch_prepare<Q, S>(m, s);
+  }
+  if (rc) return rc;
+  for (int64_t i = 0; i + 1 < n; ++i) {
+    m.pin = A;
+    m.pout = B;
+    rc = launch_state_step<Q, S>(p, m, s);
+    if (rc) return rc;
+    char* t = A;
+    A = B;
+    B = t;
+  }
+  a.pin = A;
+  a.f_out = f_out;
+  return launch_step<Q, S>(a, true, s);
+}
+
+// Rollout that also records the reference state after every `every`-th step
+// (record r = after step (r + 1) every): recorded state steps write f and the
+// moments into the history slots as they collide; the last step's outputs are
+// copied into its slot when it is recorded.
+template <int Q, class S>
+int run_history(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in,
+                void* f_out, int64_t n, int64_t every, const lbm_history* h, char* ws) {
+  const size_t sb = align256(state_bytes(p));
+  const size_t cells = p->g.ncell;
+  const size_t fb = cells * p->Q * p->io, rb = cells * p->io, vb = cells * p->D * p->io;
+  auto slot = [](void* base, size_t bytes, int64_t r) -> void* {
+    return base == nullptr ? nullptr : static_cast<char*>(base) + static_cast<size_t>(r) * bytes;
+  };
+  char* A = ws;
+  char* B = ws + sb;
+  lbm::StepArgs m = a;
+  m.rho = m.vel = m.prs = nullptr;
+  m.f_in = f_in;
+  m.pout = A;
+  int rc = launch_prepare<Q, S>(m, s);
+  if (rc) return rc;
+  for (int64_t i = 1; i < n; ++i) {
+    m.pin = A;
+    m.pout = B;
+    if (i % every == 0) {
+      const int64_t r = i / every - 1;
+      lbm::StepArgs rec = m;
+      rec.f_out = slot(h->f, fb, r);
+      rec.rho = slot(h->density, rb, r);
+      rec.vel = slot(h->velocity, vb, r);
+      rec.prs = slot(h->pressure, rb, r);
+      launch_step_mode<Q, S, lbm::kOutRecord>(rec, s);
+      rc = cuda_check(cudaGetLastError(), "k_step launch");
+    } else {
+      rc = launch_state_step<Q, S>(p, m, s);
+    }
+    if (rc) return rc;
+    char* t = A;
+    A = B;
+    B = t;
+  }
+  const bool last = n % every == 0;
+  const int64_t r = n / every - 1;
+  a.pin = A;
+  a.f_out = f_out;
+  // the last step's moments go to the caller's buffers, or straight to the
+  // history slot when the caller wants none
+  if (last && a.rho == nullptr) a.rho = slot(h->density, rb, r);
+  if (last && a.vel == nullptr) a.vel = slot(h->velocity, vb, r);
+  if (last && a.prs == nullptr) a.prs = slot(h->pressure, rb, r);
+  rc = launch_step<Q, S>(a, true, s);
+  if (rc || !last) return rc;
+  struct { void* dst; const void* src; size_t bytes; } copies[4] = {
+      {slot(h->f, fb, r), f_out, fb},
+      {slot(h->density, rb, r), a.rho, rb},
+      {slot(h->velocity, vb, r), a.vel, vb},
+      {slot(h->pressure, rb, r), a.prs, rb}};
+  for (const auto& c : copies) {
+    if (c.dst == nullptr || c.dst == c.src) continue;
+    rc = cuda_check(cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToDevice, s),
+                    "cudaMemcpyAsync");
+    if (rc) return rc;
+  }
+  return LBM_OK;
+}
+
+template <int Q, class S>
+int state_op(StateOp op, const lbm::StepArgs& a, cudaStream_t s) {
+  if (op == kFromF) return launch_prepare<Q, S>(a, s);
+  if (op == kStep) {
+    launch_step_mode<Q, S, lbm::kOutState>(a, s);  // one cell per thread, any storage
+    return cuda_check(cudaGetLastError(), "k_step launch");
+  }
+  return launch_step<Q, S>(a, true, s);
+}
+
+#define LBM_UNIT(Q, S)                                                                        \
+  template int launch_prepare<Q, S>(const lbm::StepArgs&, cudaStream_t);                      \
+  template int launch_step<Q, S>(const lbm::StepArgs&, bool, cudaStream_t);                   \
+  template int launch_step_moments_only<Q, S>(const lbm::StepArgs&, cudaStream_t);            \
+  template int launch_state_step<Q, S>(const lbm_plan*, const lbm::StepArgs&, cudaStream_t);  \
+  template int run_padded<Q, S>(const lbm_plan*, cudaStream_t, lbm::StepArgs, const void*,    \
+                                void*, char*);                                                \
+  template int run_steps<Q, S>(const lbm_plan*, cudaStream_t, lbm::StepArgs, const void*,     \
+                               void*, int64_t, char*);                                        \
+  template int run_history<Q, S>(const lbm_plan*, cudaStream_t, lbm::StepArgs, const void*,   \
+                                 void*, int64_t, int64_t, const lbm_history*, char*);         \
+  template int state_op<Q, S>(StateOp, const lbm::StepArgs&, cudaStream_t);
+LBM_UNIT(LBM_UNIT_Q, LBM_UNIT_S)

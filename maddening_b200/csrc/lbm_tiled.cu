@@ -83,9 +83,4 @@ int launch_tiled(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s) {
                                                 cudaStream_t);                           \
   template int launch_tiled<Q, S, lbm::kOutState>(const lbm_plan*, const lbm::StepArgs&, \
                                                   cudaStream_t);
-LBM_TILED_INST(19, float)
-LBM_TILED_INST(19, __half)
-LBM_TILED_INST(19, __nv_bfloat16)
-LBM_TILED_INST(9, float)
-LBM_TILED_INST(9, __half)
-LBM_TILED_INST(9, __nv_bfloat16)
+LBM_TILED_INST(LBM_UNIT_Q, LBM_UNIT_S)
