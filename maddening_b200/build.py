@@ -33,7 +33,7 @@ HEADERS = ["lbm_host.h", "lbm_kernels.cuh", "lbm_lattice.cuh", "lbm_adjoint.cuh"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CFLAGS = ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
-          "-Xcompiler", "-fPIC,-O3"]
+          "-Xcompiler", "-fPIC,-O3", "-Xfatbin", "-compress-all"]
 # Units: (source, object name, definitions).  The step kernels are compiled once
 # per lattice and storage, side by side, and each unit as a whole: a split
 # compile of one large unit gave code that differed from build to build, with

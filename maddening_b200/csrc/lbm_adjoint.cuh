@@ -140,7 +140,7 @@ __device__ __forceinline__ void adj_cell(const AdjArgs& a, uint32_t cidx) {
     nu[q] = ld_pop<S>(static_cast<const S*>(a.min) + (static_cast<uint32_t>(q) * g.ncell + off));
   }
 
-  const bool wall = a.wall != nullptr && __ldg(a.wall + cidx) != 0;
+  const bool wall = a.wall != nullptr && ld_now(a.wall + cidx) != 0;
   const R rho = static_cast<R>(static_cast<const IO*>(a.rho)[cidx]);
   R u[3] = {0, 0, 0};
 #pragma unroll
@@ -230,7 +230,9 @@ __device__ __forceinline__ void adj_cell(const AdjArgs& a, uint32_t cidx) {
 template <int Q, class S, bool FORCE, int MODE>
 __global__ void __launch_bounds__(kBlock, min_blocks<S>()) k_adj_step(const AdjArgs a) {
   using IO = typename StoreT<S>::IO;
+  grid_launch_next();
   const uint32_t cidx = blockIdx.x * kBlock + threadIdx.x;
+  grid_wait_previous();
   if (cidx < a.g.ncell) adj_cell<Q, S, FORCE, MODE>(a, cidx);
   if constexpr (MODE == kAdjOutAoS)
     aos_flush<Q, IO>(static_cast<IO*>(a.grad_f0), blockIdx.x * kBlock, a.g.ncell);

@@ -158,11 +158,11 @@ int adj_backward(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void*
       const bool aos = n == 0 && grad_f_in != nullptr;
       q.grad_f0 = grad_f_in;
       if (aos) {
-        if (force) lbm::k_adj_step<Q, S, true, lbm::kAdjOutAoS><<<grid, lbm::kBlock, 0, s>>>(q);
-        else lbm::k_adj_step<Q, S, false, lbm::kAdjOutAoS><<<grid, lbm::kBlock, 0, s>>>(q);
+        if (force) launch_after(lbm::k_adj_step<Q, S, true, lbm::kAdjOutAoS>, grid, lbm::kBlock, s, q);
+        else launch_after(lbm::k_adj_step<Q, S, false, lbm::kAdjOutAoS>, grid, lbm::kBlock, s, q);
       } else {
-        if (force) lbm::k_adj_step<Q, S, true, lbm::kAdjOutState><<<grid, lbm::kBlock, 0, s>>>(q);
-        else lbm::k_adj_step<Q, S, false, lbm::kAdjOutState><<<grid, lbm::kBlock, 0, s>>>(q);
+        if (force) launch_after(lbm::k_adj_step<Q, S, true, lbm::kAdjOutState>, grid, lbm::kBlock, s, q);
+        else launch_after(lbm::k_adj_step<Q, S, false, lbm::kAdjOutState>, grid, lbm::kBlock, s, q);
       }
       rc = cuda_check(cudaGetLastError(), "k_adj_step launch");
       if (rc) return rc;

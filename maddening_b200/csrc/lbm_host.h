@@ -37,6 +37,24 @@ inline size_t state_bytes(const lbm_plan* p) {
 
 inline unsigned grid_for(uint64_t n) { return static_cast<unsigned>((n + lbm::kBlock - 1) / lbm::kBlock); }
 
+// Launches a kernel whose blocks may start while the kernel before it in the
+// stream is still finishing (programmatic stream serialisation): only for
+// kernels that call grid_wait_previous() before their first memory access.
+template <class... KA, class... A>
+cudaError_t launch_after(void (*kern)(KA...), dim3 grid, unsigned block, cudaStream_t s,
+                         const A&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // ---- Launchers, one unit per lattice and storage (lbm_steps.cu) ----------
 // p = C(f) of the reference state a.f_in into a.pout.
 template <int Q, class S>

@@ -134,7 +134,7 @@ __device__ __forceinline__ void mp_pull(const MPArgs& a, const MPNbr& o, uint32_
   const R* fi = static_cast<const R*>(a.fin);
   const uint32_t n = a.s.g.ncell;
 #pragma unroll
-  for (int q = 0; q < 19; ++q) f[q] = __ldg(fi + static_cast<size_t>(q) * n + mp_at(o, c, q, -1));
+  for (int q = 0; q < 19; ++q) f[q] = ld_now(fi + static_cast<size_t>(q) * n + mp_at(o, c, q, -1));
 }
 
 // The floor of lbm_pipe.py:838-848 on the pulled populations f (sum s0):
@@ -190,8 +190,10 @@ __device__ __forceinline__ void density_cell(const MPArgs& a, uint32_t c, R (&f)
 
 template <class R, int MODE>
 __global__ void __launch_bounds__(kBlock) k_mp_density(const MPArgs a) {
+  grid_launch_next();
   const Geo& g = a.s.g;
   const uint32_t c = blockIdx.x * kBlock + threadIdx.x;
+  grid_wait_previous();
   R f[19];
   // the first and last passes stage the reference layout: every thread of
   // the block reaches the tile's barriers
@@ -218,8 +220,10 @@ __global__ void __launch_bounds__(kBlock) k_mp_density(const MPArgs a) {
 // f_bc (staged tile), no floor.
 template <class R, bool FIRST>
 __global__ void __launch_bounds__(kBlock) k_mp_collide(const MPArgs a) {
+  grid_launch_next();
   const Geo& g = a.s.g;
   const uint32_t c = blockIdx.x * kBlock + threadIdx.x;
+  grid_wait_previous();
   R f[19];
   const R* row = nullptr;
   if constexpr (FIRST)
@@ -231,9 +235,9 @@ __global__ void __launch_bounds__(kBlock) k_mp_collide(const MPArgs a) {
   // that they travel with the population loads (only fluid cells use them)
   const R* psi = static_cast<const R*>(a.psi);
   R pn[19];
-  pn[0] = __ldg(psi + c);
+  pn[0] = ld_now(psi + c);
 #pragma unroll
-  for (int q = 1; q < 19; ++q) pn[q] = __ldg(psi + mp_at(o, c, q, 1));
+  for (int q = 1; q < 19; ++q) pn[q] = ld_now(psi + mp_at(o, c, q, 1));
   const uint8_t* wm = a.s.wall;
   const bool wall = wm != nullptr && wm[c] != 0;
   R rho;

@@ -45,7 +45,7 @@ template <>
 struct PairT<__half> {
   using P = uint32_t;
   static __device__ __forceinline__ P ld(const __half* p) {
-    return __ldg(reinterpret_cast<const unsigned int*>(p));
+    return ld_now(reinterpret_cast<const unsigned int*>(p));
   }
   static __device__ __forceinline__ float lo(P v) {
     return __low2float(*reinterpret_cast<const __half2*>(&v));
@@ -59,7 +59,7 @@ template <>
 struct PairT<__nv_bfloat16> {
   using P = uint32_t;
   static __device__ __forceinline__ P ld(const __nv_bfloat16* p) {
-    return __ldg(reinterpret_cast<const unsigned int*>(p));
+    return ld_now(reinterpret_cast<const unsigned int*>(p));
   }
   static __device__ __forceinline__ float lo(P v) { return __uint_as_float(v << 16); }
   static __device__ __forceinline__ float hi(P v) { return __uint_as_float(v & 0xffff0000u); }
@@ -69,7 +69,7 @@ template <>
 struct PairT<float> {
   using P = float2;
   static __device__ __forceinline__ P ld(const float* p) {
-    return __ldg(reinterpret_cast<const float2*>(p));
+    return ld_now(reinterpret_cast<const float2*>(p));
   }
   static __device__ __forceinline__ float lo(P v) { return v.x; }
   static __device__ __forceinline__ float hi(P v) { return v.y; }
@@ -147,10 +147,10 @@ __device__ __forceinline__ void pair_finish(const StepArgs& a, uint32_t i0, uint
   bool wa = false, wb = false;
   if (a.wall != nullptr) {
     if constexpr (PAD) {  // odd rows: the two wall bytes are not 2-byte aligned
-      wa = __ldg(a.wall + rbase + k) != 0;
-      wb = !last && __ldg(a.wall + rbase + k + 1) != 0;
+      wa = ld_now(a.wall + rbase + k) != 0;
+      wb = !last && ld_now(a.wall + rbase + k + 1) != 0;
     } else {
-      const uint32_t w2 = __ldg(reinterpret_cast<const unsigned short*>(a.wall + rbase + k));
+      const uint32_t w2 = ld_now(reinterpret_cast<const unsigned short*>(a.wall + rbase + k));
       wa = (w2 & 0xffu) != 0;
       wb = (w2 >> 8) != 0;
     }
@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(32 * W, kPairMinWarps / W)
     k_step_pair(const __grid_constant__ StepArgs a) {
   using PT = PairT<S>;
   using P = typename PT::P;
+  grid_launch_next();
   const Geo& g = a.g;
   const uint32_t row = blockIdx.x;
   const uint32_t i0 = fdiv(row, g.div_n1);
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(32 * W, kPairMinWarps / W)
   const uint32_t i0m = i0 == 0 ? g.n0 - 1 : i0 - 1, i0p = i0 + 1 == g.n0 ? 0u : i0 + 1;
   const uint32_t i1m = i1 == 0 ? g.n1 - 1 : i1 - 1, i1p = i1 + 1 == g.n1 ? 0u : i1 + 1;
 
+  grid_wait_previous();
   const S* pin = static_cast<const S*>(a.pin);
   P v[Q];
   P e[Q];
@@ -252,7 +254,7 @@ __global__ void __launch_bounds__(32 * W, kPairMinWarps / W)
 template <class S>
 struct QuadT {
   static __device__ __forceinline__ uint2 ld(const S* p) {
-    return __ldg(reinterpret_cast<const uint2*>(p));
+    return ld_now(reinterpret_cast<const uint2*>(p));
   }
 };
 
@@ -308,7 +310,7 @@ __device__ __forceinline__ void quad_finish(const StepArgs& a, uint32_t i0, uint
   const uint32_t rbase = row * g.n2, sbase = row * g.rstride;
   bool w[4] = {false, false, false, false};
   if (a.wall != nullptr) {
-    const uint32_t w4 = __ldg(reinterpret_cast<const unsigned int*>(a.wall + rbase + k));
+    const uint32_t w4 = ld_now(reinterpret_cast<const unsigned int*>(a.wall + rbase + k));
 #pragma unroll
     for (int j = 0; j < 4; ++j) w[j] = ((w4 >> (8 * j)) & 0xffu) != 0;
   }
@@ -366,6 +368,7 @@ __device__ __forceinline__ void quad_finish(const StepArgs& a, uint32_t i0, uint
 template <int Q, class S, bool FACES, bool FORCE, int W>
 __global__ void __launch_bounds__(32 * W, quad_min_warps<Q>() / W)
     k_step_quad(const __grid_constant__ StepArgs a) {
+  grid_launch_next();
   const Geo& g = a.g;
   const uint32_t row = blockIdx.x;
   const uint32_t i0 = fdiv(row, g.div_n1);
@@ -375,6 +378,7 @@ __global__ void __launch_bounds__(32 * W, quad_min_warps<Q>() / W)
   const uint32_t knext = k + 4u == g.n2 ? 0u : k + 4u;  // word holding cell k + 4 (low)
   const uint32_t i0m = i0 == 0 ? g.n0 - 1 : i0 - 1, i0p = i0 + 1 == g.n0 ? 0u : i0 + 1;
   const uint32_t i1m = i1 == 0 ? g.n1 - 1 : i1 - 1, i1p = i1 + 1 == g.n1 ? 0u : i1 + 1;
+  grid_wait_previous();
   const S* pin = static_cast<const S*>(a.pin);
   float d[4][Q];
 #pragma unroll
@@ -394,6 +398,7 @@ __global__ void __launch_bounds__(32 * W, quad_min_warps<Q>() / W)
 template <int Q, class S, bool FACES, bool FORCE>
 __global__ void __launch_bounds__(kBlock, quad_min_warps<Q>() / (kBlock / 32))
     k_step_gquad(const __grid_constant__ StepArgs a) {
+  grid_launch_next();
   const Geo& g = a.g;
   const uint32_t nquads = g.ncell >> 2;
   const uint32_t qidx = blockIdx.x * kBlock + threadIdx.x;
@@ -407,6 +412,7 @@ __global__ void __launch_bounds__(kBlock, quad_min_warps<Q>() / (kBlock / 32))
   const uint32_t knext = k + 4u == g.n2 ? 0u : k + 4u;
   const uint32_t i0m = i0 == 0 ? g.n0 - 1 : i0 - 1, i0p = i0 + 1 == g.n0 ? 0u : i0 + 1;
   const uint32_t i1m = i1 == 0 ? g.n1 - 1 : i1 - 1, i1p = i1 + 1 == g.n1 ? 0u : i1 + 1;
+  grid_wait_previous();
   const S* pin = static_cast<const S*>(a.pin);
   float d[4][Q];
 #pragma unroll
@@ -469,6 +475,8 @@ __device__ __forceinline__ void gpair_step(const StepArgs& a, uint32_t pidx) {
 template <int Q, class S, bool FACES, bool FORCE>
 __global__ void __launch_bounds__(kBlock, kGPairMinWarps / (kBlock / 32))
     k_step_gpair(const __grid_constant__ StepArgs a) {
+  grid_launch_next();
+  grid_wait_previous();
   gpair_step<Q, S, FACES, FORCE, false>(a, blockIdx.x * kBlock + threadIdx.x);
 }
 
@@ -479,22 +487,11 @@ template <int Q, class S, int SPEC, bool PAD>
 __global__ void __launch_bounds__(kBlock, kGPairMinWarps / (kBlock / 32))
     k_batched_pair(const StepArgs* __restrict__ args, const BatchTile* __restrict__ tiles,
                    uint32_t ntiles, int which) {
-#if LBM_BATCH_ARGS_SMEM
-  __shared__ StepArgs sa;
-  uint32_t cur = 0xffffffffu;
-#endif
+  grid_launch_next();
+  grid_wait_previous();
   for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const BatchTile tile = tiles[t];
-#if LBM_BATCH_ARGS_SMEM
-    if (tile.inst != cur) {
-      __syncthreads();
-      stage_args(sa, args[kBatchArgs * tile.inst + which]);
-      __syncthreads();
-      cur = tile.inst;
-    }
-#else
     const StepArgs& sa = args[kBatchArgs * tile.inst + which];
-#endif
 #pragma unroll 1
     for (int j = 0; j < kBatchTile / (2 * kBlock); ++j) {
       const uint32_t pidx = (tile.first >> 1) + j * kBlock + threadIdx.x;

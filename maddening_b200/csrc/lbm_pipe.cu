@@ -43,7 +43,7 @@ int run_pipe(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_i
     m.pout = B;
     t.tin = T[cur];
     t.tout = T[1 - cur];
-    lbm::k_pipe_step<S, false><<<grid, lbm::kBlock, 0, s>>>(m, t);
+    launch_after(lbm::k_pipe_step<S, false>, grid, lbm::kBlock, s, m, t);
     rc = cuda_check(cudaGetLastError(), "k_pipe_step launch");
     if (rc) return rc;
     cur = 1 - cur;
@@ -55,14 +55,14 @@ int run_pipe(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_i
   a.mflags &= ~lbm::kMomRawVelocity;
   t.tin = T[cur];
   t.tout = T[1 - cur];
-  lbm::k_pipe_step<S, true><<<grid, lbm::kBlock, 0, s>>>(a, t);
+  launch_after(lbm::k_pipe_step<S, true>, grid, lbm::kBlock, s, a, t);
   rc = cuda_check(cudaGetLastError(), "k_pipe_step launch");
   if (rc) return rc;
   cur = 1 - cur;
   t.tin = T[cur];
   t.f7_out = t_out;
   t.tracer_out = tracer_out;
-  lbm::k_tracer_final<IO><<<grid, lbm::kBlock, 0, s>>>(t);
+  launch_after(lbm::k_tracer_final<IO>, grid, lbm::kBlock, s, t);
   return cuda_check(cudaGetLastError(), "k_tracer_final launch");
 }
 
@@ -88,21 +88,21 @@ int run_pipe_mp(const lbm_plan* p, cudaStream_t s, const lbm::StepArgs& a,
   m.f_aos_in = f_in;
   const unsigned grid = grid_for(p->g.ncell);
   // step 1: psi of the reference f, then its collide into A
-  lbm::k_mp_density<R, lbm::kMPFirst><<<grid, lbm::kBlock, 0, s>>>(m);
+  launch_after(lbm::k_mp_density<R, lbm::kMPFirst>, grid, lbm::kBlock, s, m);
   int rc = cuda_check(cudaGetLastError(), "k_mp_density launch");
   if (rc) return rc;
   m.fout = A;
-  lbm::k_mp_collide<R, true><<<grid, lbm::kBlock, 0, s>>>(m);
+  launch_after(lbm::k_mp_collide<R, true>, grid, lbm::kBlock, s, m);
   rc = cuda_check(cudaGetLastError(), "k_mp_collide launch");
   if (rc) return rc;
   // steps 2..n: both passes pull from the post-collision planes
   for (int64_t i = 1; i < n; ++i) {
     m.fin = A;
     m.fout = B;
-    lbm::k_mp_density<R, lbm::kMPStep><<<grid, lbm::kBlock, 0, s>>>(m);
+    launch_after(lbm::k_mp_density<R, lbm::kMPStep>, grid, lbm::kBlock, s, m);
     rc = cuda_check(cudaGetLastError(), "k_mp_density launch");
     if (rc) return rc;
-    lbm::k_mp_collide<R, false><<<grid, lbm::kBlock, 0, s>>>(m);
+    launch_after(lbm::k_mp_collide<R, false>, grid, lbm::kBlock, s, m);
     rc = cuda_check(cudaGetLastError(), "k_mp_collide launch");
     if (rc) return rc;
     std::swap(A, B);
@@ -112,7 +112,7 @@ int run_pipe_mp(const lbm_plan* p, cudaStream_t s, const lbm::StepArgs& a,
   m.rho_out = out != nullptr ? out->density : nullptr;
   m.vel_out = out != nullptr ? out->velocity : nullptr;
   m.tracer_out = tracer_out;
-  lbm::k_mp_density<R, lbm::kMPLast><<<grid, lbm::kBlock, 0, s>>>(m);
+  launch_after(lbm::k_mp_density<R, lbm::kMPLast>, grid, lbm::kBlock, s, m);
   rc = cuda_check(cudaGetLastError(), "k_mp_density launch");
   if (rc) return rc;
   // tracer_f is not evolved in multiphase mode (lbm_pipe.py:858-860)

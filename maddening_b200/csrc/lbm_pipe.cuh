@@ -94,12 +94,14 @@ __global__ void __launch_bounds__(kBlock, min_blocks<S>())
     k_pipe_step(const __grid_constant__ StepArgs a, const __grid_constant__ TracerArgs t) {
   using R = typename StoreT<S>::R;
   using IO = typename StoreT<S>::IO;
+  grid_launch_next();
   const uint32_t cidx = blockIdx.x * kBlock + threadIdx.x;
+  grid_wait_previous();
   if (cidx < a.g.ncell) {
     const Cell x = locate(a.g, cidx);
     R d[19];
     pull_cell<19, S>(a, x, d);
-    const bool wall = a.wall != nullptr && __ldg(a.wall + cidx) != 0;
+    const bool wall = a.wall != nullptr && ld_now(a.wall + cidx) != 0;
     R F[3];
     pipe_force<R>(a, cidx, wall, F);
     apply_bc<19, S, false>(a, x, wall, d);
@@ -127,6 +129,7 @@ __global__ void __launch_bounds__(kBlock, min_blocks<S>())
 // Last pass: populations to the reference layout and the tracer field.
 template <class IO>
 __global__ void __launch_bounds__(kBlock) k_tracer_final(const TracerArgs a) {
+  grid_wait_previous();
   const uint32_t c = blockIdx.x * kBlock + threadIdx.x;
   if (c < a.g.ncell) {
     const IO* tin = static_cast<const IO*>(a.tin);

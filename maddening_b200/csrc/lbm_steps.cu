@@ -15,11 +15,11 @@ void launch_step_mode(const lbm::StepArgs& a, cudaStream_t s) {
   const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
   const bool force = a.force_mode != 0;
   if (faces) {
-    if (force) lbm::k_step<Q, S, MODE, true, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step<Q, S, MODE, true, false><<<grid, lbm::kBlock, 0, s>>>(a);
+    if (force) launch_after(lbm::k_step<Q, S, MODE, true, true>, grid, lbm::kBlock, s, a);
+    else launch_after(lbm::k_step<Q, S, MODE, true, false>, grid, lbm::kBlock, s, a);
   } else {
-    if (force) lbm::k_step<Q, S, MODE, false, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step<Q, S, MODE, false, false><<<grid, lbm::kBlock, 0, s>>>(a);
+    if (force) launch_after(lbm::k_step<Q, S, MODE, false, true>, grid, lbm::kBlock, s, a);
+    else launch_after(lbm::k_step<Q, S, MODE, false, false>, grid, lbm::kBlock, s, a);
   }
 }
 
@@ -48,11 +48,11 @@ void launch_pair_w(const lbm::StepArgs& a, cudaStream_t s) {
   const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
   const bool force = a.force_mode != 0;
   if (faces) {
-    if (force) lbm::k_step_pair<Q, S, true, true, W><<<grid, 32 * W, 0, s>>>(a);
-    else lbm::k_step_pair<Q, S, true, false, W><<<grid, 32 * W, 0, s>>>(a);
+    if (force) launch_after(lbm::k_step_pair<Q, S, true, true, W>, grid, 32 * W, s, a);
+    else launch_after(lbm::k_step_pair<Q, S, true, false, W>, grid, 32 * W, s, a);
   } else {
-    if (force) lbm::k_step_pair<Q, S, false, true, W><<<grid, 32 * W, 0, s>>>(a);
-    else lbm::k_step_pair<Q, S, false, false, W><<<grid, 32 * W, 0, s>>>(a);
+    if (force) launch_after(lbm::k_step_pair<Q, S, false, true, W>, grid, 32 * W, s, a);
+    else launch_after(lbm::k_step_pair<Q, S, false, false, W>, grid, 32 * W, s, a);
   }
 }
 
@@ -62,11 +62,11 @@ void launch_quad_w(const lbm::StepArgs& a, cudaStream_t s) {
   const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
   const bool force = a.force_mode != 0;
   if (faces) {
-    if (force) lbm::k_step_quad<Q, S, true, true, W><<<grid, 32 * W, 0, s>>>(a);
-    else lbm::k_step_quad<Q, S, true, false, W><<<grid, 32 * W, 0, s>>>(a);
+    if (force) launch_after(lbm::k_step_quad<Q, S, true, true, W>, grid, 32 * W, s, a);
+    else launch_after(lbm::k_step_quad<Q, S, true, false, W>, grid, 32 * W, s, a);
   } else {
-    if (force) lbm::k_step_quad<Q, S, false, true, W><<<grid, 32 * W, 0, s>>>(a);
-    else lbm::k_step_quad<Q, S, false, false, W><<<grid, 32 * W, 0, s>>>(a);
+    if (force) launch_after(lbm::k_step_quad<Q, S, false, true, W>, grid, 32 * W, s, a);
+    else launch_after(lbm::k_step_quad<Q, S, false, false, W>, grid, 32 * W, s, a);
   }
 }
 
@@ -94,11 +94,11 @@ void launch_gquad(const lbm::StepArgs& a, cudaStream_t s) {
   const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
   const bool force = a.force_mode != 0;
   if (faces) {
-    if (force) lbm::k_step_gquad<Q, S, true, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step_gquad<Q, S, true, false><<<grid, lbm::kBlock, 0, s>>>(a);
+    if (force) launch_after(lbm::k_step_gquad<Q, S, true, true>, grid, lbm::kBlock, s, a);
+    else launch_after(lbm::k_step_gquad<Q, S, true, false>, grid, lbm::kBlock, s, a);
   } else {
-    if (force) lbm::k_step_gquad<Q, S, false, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step_gquad<Q, S, false, false><<<grid, lbm::kBlock, 0, s>>>(a);
+    if (force) launch_after(lbm::k_step_gquad<Q, S, false, true>, grid, lbm::kBlock, s, a);
+    else launch_after(lbm::k_step_gquad<Q, S, false, false>, grid, lbm::kBlock, s, a);
   }
 }
 
@@ -122,11 +122,11 @@ void launch_gpair(const lbm::StepArgs& a, cudaStream_t s) {
   const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
   const bool force = a.force_mode != 0;
   if (faces) {
-    if (force) lbm::k_step_gpair<Q, S, true, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step_gpair<Q, S, true, false><<<grid, lbm::kBlock, 0, s>>>(a);
+    if (force) launch_after(lbm::k_step_gpair<Q, S, true, true>, grid, lbm::kBlock, s, a);
+    else launch_after(lbm::k_step_gpair<Q, S, true, false>, grid, lbm::kBlock, s, a);
   } else {
-    if (force) lbm::k_step_gpair<Q, S, false, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step_gpair<Q, S, false, false><<<grid, lbm::kBlock, 0, s>>>(a);
+    if (force) launch_after(lbm::k_step_gpair<Q, S, false, true>, grid, lbm::kBlock, s, a);
+    else launch_after(lbm::k_step_gpair<Q, S, false, false>, grid, lbm::kBlock, s, a);
   }
 }
 
@@ -163,11 +163,11 @@ int launch_step_padded(const lbm::StepArgs& a, cudaStream_t s) {
   const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
   const bool force = a.force_mode != 0;
   if (faces) {
-    if (force) lbm::k_step_padded<Q, S, true, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step_padded<Q, S, true, false><<<grid, lbm::kBlock, 0, s>>>(a);
+    if (force) launch_after(lbm::k_step_padded<Q, S, true, true>, grid, lbm::kBlock, s, a);
+    else launch_after(lbm::k_step_padded<Q, S, true, false>, grid, lbm::kBlock, s, a);
   } else {
-    if (force) lbm::k_step_padded<Q, S, false, true><<<grid, lbm::kBlock, 0, s>>>(a);
-    else lbm::k_step_padded<Q, S, false, false><<<grid, lbm::kBlock, 0, s>>>(a);
+    if (force) launch_after(lbm::k_step_padded<Q, S, false, true>, grid, lbm::kBlock, s, a);
+    else launch_after(lbm::k_step_padded<Q, S, false, false>, grid, lbm::kBlock, s, a);
   }
   return cuda_check(cudaGetLastError(), "k_step_padded launch");
 }
