@@ -20,9 +20,9 @@
 //            loads the same line, so it hits L1); cell k+1 reads the low half
 //            of its own pair;
 //   c2 = -1: mirror image (the pair after, wrapped at the row end).
-// After the pull each cell runs exactly the arithmetic of the one-cell step
-// (wall swap -> faces -> moments -> collide), so the results are
-// bit-identical; the wall swap is skipped by warps without a wall cell and the
+// After the pull both cells run the arithmetic of the one-cell step (wall swap ->
+// faces -> moments -> collide) as two-wide FP32 operations, each half rounded
+// like the scalar one, so the results are bit-identical; the wall swap is skipped by warps without a wall cell and the
 // face checks by pairs that cannot touch a face.
 //
 // A second form (k_step_gpair) takes any even row length: pairs follow the
@@ -78,37 +78,67 @@ struct PairT<float> {
   }
 };
 
-// Resident warps per SM the register budgets are set for (a B200 sweep of
-// 20-32: the row-segment form is fastest at 32 warps despite a few spilled
-// registers, the instance-wide form at 28).
-#ifndef LBM_PAIR_MIN_WARPS
-#define LBM_PAIR_MIN_WARPS 32
-#endif
-#ifndef LBM_GPAIR_MIN_WARPS
-#define LBM_GPAIR_MIN_WARPS 28
-#endif
-constexpr int kPairMinWarps = LBM_PAIR_MIN_WARPS;
-constexpr int kGPairMinWarps = LBM_GPAIR_MIN_WARPS;
+// Resident warps per SM the register budgets are set for.  With two-wide
+// arithmetic the pair holds its values in register pairs: 24 warps (80 registers)
+// beat 28 and 32, which spill (B200, FP16 / BF16 with a force: 128^3 rows 32.7 us
+// a step against 35.0 at 32 and 38.0 with one-wide arithmetic; 250^3 229.9 /
+// 245.7 / 252.5; 149 x 111 x 94 26.7 / 26.0 / 30.8), and 20 and 16 (34.0, 35.8 us
+// at 128^3).
+constexpr int kPairMinWarps = 24;
 
-// Moments and collide of one cell whose f_bc populations are in d; `real` =
-// false for the padding cell of a padded row (its result is never read).
-// Returns the cell's stochastic-rounding seed (16-bit storage; else 0).
+// Wall-node swap of the cells of a pair (w0: low half, w1: high half).
+template <int Q>
+__device__ __forceinline__ void wall_swap2(F2 (&d)[Q], bool w0, bool w1) {
+#pragma unroll
+  for (int q = 1; q < Q; ++q) {
+    const int o = Lat<Q>::opp(q);
+    if (q > o) continue;
+    const F2 x = d[q], y = d[o];
+    d[q] = F2(w0 ? y.v.x : x.v.x, w1 ? y.v.y : x.v.y);
+    d[o] = F2(w0 ? x.v.x : y.v.x, w1 ? x.v.y : y.v.y);
+  }
+}
+
+// Faces of one cell of a pair (HI: the high half).
+template <int Q, class S, bool HI>
+__device__ __forceinline__ void apply_faces2(const StepArgs& a, const Cell& x, F2 (&d)[Q]) {
+  float t[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) t[q] = HI ? d[q].v.y : d[q].v.x;
+  apply_faces<Q, S>(a, x, t);
+#pragma unroll
+  for (int q = 0; q < Q; ++q) d[q] = HI ? F2(d[q].v.x, t[q]) : F2(t[q], d[q].v.y);
+}
+
+// Moments and collide of two neighbouring cells c, c + 1 whose f_bc populations
+// are in d; `real1` = false where cell c + 1 is the padding cell of a padded
+// row (its result is never read).  Returns the pair's stochastic-rounding
+// seeds (16-bit storage; else 0).
 template <int Q, class S, bool FORCE>
-__device__ __forceinline__ uint32_t pair_cell(const StepArgs& a, const Cell& x, float (&d)[Q],
-                                              bool real = true) {
+__device__ __forceinline__ uint32_t pair_cells(const StepArgs& a, uint32_t c, F2 (&d)[Q],
+                                               bool real1 = true) {
   using IO = typename StoreT<S>::IO;
-  float F[3] = {0, 0, 0};
+  F2 F[3] = {0, 0, 0};
   if (FORCE) {
+    float F0[3] = {0, 0, 0}, F1[3] = {0, 0, 0};
     if (a.force_mode == 2) {
-      if (real) load_force<Q, IO>(a.force_field, x.c, F);
+      load_force<Q, IO>(a.force_field, c, F0);
+      if (real1) load_force<Q, IO>(a.force_field, c + 1, F1);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) F[k] = F2(F0[k], F1[k]);
     } else {
-      uniform_force<Q, float>(a, F);
+      uniform_force<Q, float>(a, F0);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) F[k] = F2(F0[k]);
     }
   }
-  const Mom<float> m = moments<Q, float, FORCE>(d, F);
-  collide<Q, float, FORCE>(d, m, F, static_cast<float>(a.omega), static_cast<float>(a.guo_c));
-  if constexpr (sizeof(S) == 2) return sr_seed(x.c, m.u[0], m.u[1], m.u[2], m.rd);
-  else return 0u;
+  const Mom<F2> m = moments<Q, F2, FORCE>(d, F);
+  collide<Q, F2, FORCE>(d, m, F, F2(a.omega), F2(a.guo_c));
+  if constexpr (sizeof(S) == 2)
+    return sr_pair(sr_seed(c, m.u[0].v.x, m.u[1].v.x, m.u[2].v.x, m.rd.v.x),
+                   sr_seed(c + 1, m.u[0].v.y, m.u[1].v.y, m.u[2].v.y, m.rd.v.y));
+  else
+    return 0u;
 }
 
 // Everything after the plane loads of one thread's pair (k, k+1) of row
@@ -129,20 +159,13 @@ __device__ __forceinline__ void pair_finish(const StepArgs& a, uint32_t i0, uint
   const Geo& g = a.g;
   const bool first = PAD && k == 0;
   const bool last = PAD && k + 1 == g.n2;  // cell b is the padding cell
-  float da[Q], db[Q];
+  F2 d[Q];
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     const int c2 = Lat<Q>::c2(q);
-    if (c2 == 0) {
-      da[q] = PT::lo(v[q]);
-      db[q] = PT::hi(v[q]);
-    } else if (c2 > 0) {
-      da[q] = first ? PT::lo(e[q]) : PT::hi(e[q]);
-      db[q] = PT::lo(v[q]);
-    } else {
-      da[q] = last ? PT::lo(e[q]) : PT::hi(v[q]);
-      db[q] = PT::lo(e[q]);
-    }
+    if (c2 == 0) d[q] = F2(PT::lo(v[q]), PT::hi(v[q]));
+    else if (c2 > 0) d[q] = F2(first ? PT::lo(e[q]) : PT::hi(e[q]), PT::lo(v[q]));
+    else d[q] = F2(last ? PT::lo(e[q]) : PT::hi(v[q]), PT::lo(e[q]));
   }
   bool wa = false, wb = false;
   if (a.wall != nullptr) {
@@ -166,10 +189,7 @@ __device__ __forceinline__ void pair_finish(const StepArgs& a, uint32_t i0, uint
   xb.c = xa.c + 1;
   xb.k = k + 1;
   // Wall swap only in warps that hold a wall cell (obstacles are clustered).
-  if (__any_sync(0xffffffffu, wa || wb)) {
-    if (wa) wall_swap<Q>(da);
-    if (wb) wall_swap<Q>(db);
-  }
+  if (__any_sync(0xffffffffu, wa || wb)) wall_swap2<Q>(d, wa, wb);
   if constexpr (FACES) {
     // Only pairs on a face plane run the face code: rows on faces of axes 0
     // and 1, the first and the last pair of a row on faces of the contiguous axis.
@@ -184,22 +204,20 @@ __device__ __forceinline__ void pair_finish(const StepArgs& a, uint32_t i0, uint
       else near |= (fc.side == 0 ? ins : g.n2 - 1 - ins) - k <= 1u;  // k or k + 1
     }
     if (near) {
-      if (!wa) apply_faces<Q, S>(a, xa, da);
-      if (!wb && !last) apply_faces<Q, S>(a, xb, db);  // never on the padding cell
+      if (!wa) apply_faces2<Q, S, false>(a, xa, d);
+      if (!wb && !last) apply_faces2<Q, S, true>(a, xb, d);  // never on the padding cell
     }
   }
-  const uint32_t sa = pair_cell<Q, S, FORCE>(a, xa, da);
-  const uint32_t sb = pair_cell<Q, S, FORCE>(a, xb, db, !last);
+  const uint32_t s2 = pair_cells<Q, S, FORCE>(a, xa.c, d, !last);
   if (!store) return;
   S* pout = static_cast<S*>(a.pout);
-  const uint32_t s2 = sr_pair(sa, sb);
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     S* dst = pout + (static_cast<uint32_t>(q) * g.pstride + sbase + k);
     if constexpr (sizeof(S) == 2)
-      *reinterpret_cast<uint32_t*>(dst) = sr_two<S>(da[q], db[q], s2);
+      *reinterpret_cast<uint32_t*>(dst) = sr_two<S>(d[q].v.x, d[q].v.y, s2);
     else
-      PT::st(dst, da[q], db[q]);
+      PT::st(dst, d[q].v.x, d[q].v.y);
   }
 }
 
@@ -258,44 +276,32 @@ struct QuadT {
   }
 };
 
-// Resident warps the D3Q19 four-cell budget is set for (B200 sweep at 256^3,
-// FP16: 16 warps 78.1k, 20 warps 79.4k, 22 / 24 warps 69k MLUPS -- at 20 the 96
-// registers spill a few bytes, beyond it the spills cost more than the warps).
-#ifndef LBM_QUAD19_MIN_WARPS
-#define LBM_QUAD19_MIN_WARPS 20
-#endif
-// D2Q9 four-cell budget (B200 sweep, 4096^2 channel FP16: 24 / 32 / 40 / 48
-// resident warps 134.9k / 138.5k / 125.0k / 98.9k MLUPS).
-#ifndef LBM_QUAD9_MIN_WARPS
-#define LBM_QUAD9_MIN_WARPS LBM_PAIR_MIN_WARPS
-#endif
-template <int Q>
-constexpr int quad_min_warps() { return Q == 19 ? LBM_QUAD19_MIN_WARPS : LBM_QUAD9_MIN_WARPS; }
+// Resident warps the four-cell budgets are set for.  D3Q19, 256^3 FP16: with a
+// force 16 warps (128 registers) 219.3 us a step, 18: 253, 20: 247.6 (239.8 with
+// one-wide arithmetic at 20); without one 20 warps 219.1, 18: 221.8, 16: 223.8
+// (227.4).  D2Q9, 4096^2 FP16 with a force: 28 warps 110.6 us, 32: 113.2, 24:
+// 114.4, 20: 122.8 (121.1 one-wide at 32).
+template <int Q, bool FORCE>
+constexpr int quad_min_warps() { return Q == 19 ? (FORCE ? 16 : 20) : 28; }
 
 // The populations of quad (k..k+3) of source row `base` pulled along the row:
 // kprev / knext the aligned 32-bit words holding cells k - 1 / k + 4
 // (periodic).
 template <int Q, class S>
 __device__ __forceinline__ void quad_pull(const S* base, int q, uint32_t k, uint32_t kprev,
-                                          uint32_t knext, float (&d)[4][Q]) {
+                                          uint32_t knext, F2 (&d)[2][Q]) {
   using PT = PairT<S>;
   const int c2 = Lat<Q>::c2(q);
   const uint2 v = QuadT<S>::ld(base + k);
   if (c2 == 0) {
-    d[0][q] = PT::lo(v.x);
-    d[1][q] = PT::hi(v.x);
-    d[2][q] = PT::lo(v.y);
-    d[3][q] = PT::hi(v.y);
+    d[0][q] = F2(PT::lo(v.x), PT::hi(v.x));
+    d[1][q] = F2(PT::lo(v.y), PT::hi(v.y));
   } else if (c2 > 0) {  // cell j pulls j - 1
-    d[0][q] = PT::hi(PT::ld(base + kprev));
-    d[1][q] = PT::lo(v.x);
-    d[2][q] = PT::hi(v.x);
-    d[3][q] = PT::lo(v.y);
+    d[0][q] = F2(PT::hi(PT::ld(base + kprev)), PT::lo(v.x));
+    d[1][q] = F2(PT::hi(v.x), PT::lo(v.y));
   } else {  // cell j pulls j + 1
-    d[0][q] = PT::hi(v.x);
-    d[1][q] = PT::lo(v.y);
-    d[2][q] = PT::hi(v.y);
-    d[3][q] = PT::lo(PT::ld(base + knext));
+    d[0][q] = F2(PT::hi(v.x), PT::lo(v.y));
+    d[1][q] = F2(PT::hi(v.y), PT::lo(PT::ld(base + knext)));
   }
 }
 
@@ -304,7 +310,7 @@ __device__ __forceinline__ void quad_pull(const S* base, int q, uint32_t k, uint
 // warp call it (vote); `store` = false for lanes that only pad the warp.
 template <int Q, class S, bool FACES, bool FORCE>
 __device__ __forceinline__ void quad_finish(const StepArgs& a, uint32_t i0, uint32_t i1,
-                                            uint32_t k, uint32_t row, float (&d)[4][Q],
+                                            uint32_t k, uint32_t row, F2 (&d)[2][Q],
                                             bool store) {
   const Geo& g = a.g;
   const uint32_t rbase = row * g.n2, sbase = row * g.rstride;
@@ -315,9 +321,8 @@ __device__ __forceinline__ void quad_finish(const StepArgs& a, uint32_t i0, uint
     for (int j = 0; j < 4; ++j) w[j] = ((w4 >> (8 * j)) & 0xffu) != 0;
   }
   if (__any_sync(0xffffffffu, w[0] || w[1] || w[2] || w[3])) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (w[j]) wall_swap<Q>(d[j]);
+    wall_swap2<Q>(d[0], w[0], w[1]);
+    wall_swap2<Q>(d[1], w[2], w[3]);
   }
   Cell x;
   x.i0 = i0;
@@ -341,32 +346,27 @@ __device__ __forceinline__ void quad_finish(const StepArgs& a, uint32_t i0, uint
         if (w[j]) continue;
         x.c = rbase + k + j;
         x.k = k + j;
-        apply_faces<Q, S>(a, x, d[j]);
+        if (j & 1) apply_faces2<Q, S, true>(a, x, d[j >> 1]);
+        else apply_faces2<Q, S, false>(a, x, d[j >> 1]);
       }
     }
   }
-  uint32_t seed[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    x.c = rbase + k + j;
-    x.k = k + j;
-    seed[j] = pair_cell<Q, S, FORCE>(a, x, d[j]);
-  }
+  const uint32_t s01 = pair_cells<Q, S, FORCE>(a, rbase + k, d[0]);
+  const uint32_t s23 = pair_cells<Q, S, FORCE>(a, rbase + k + 2, d[1]);
   if (!store) return;
   S* pout = static_cast<S*>(a.pout);
-  const uint32_t s01 = sr_pair(seed[0], seed[1]), s23 = sr_pair(seed[2], seed[3]);
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     uint2 w;
-    w.x = sr_two<S>(d[0][q], d[1][q], s01);
-    w.y = sr_two<S>(d[2][q], d[3][q], s23);
+    w.x = sr_two<S>(d[0][q].v.x, d[0][q].v.y, s01);
+    w.y = sr_two<S>(d[1][q].v.x, d[1][q].v.y, s23);
     *reinterpret_cast<uint2*>(pout + (static_cast<uint32_t>(q) * g.pstride + sbase + k)) = w;
   }
 }
 
 // Row-segment form: block = W warps = 128 W consecutive cells of one row.
 template <int Q, class S, bool FACES, bool FORCE, int W>
-__global__ void __launch_bounds__(32 * W, quad_min_warps<Q>() / W)
+__global__ void __launch_bounds__(32 * W, quad_min_warps<Q, FORCE>() / W)
     k_step_quad(const __grid_constant__ StepArgs a) {
   grid_launch_next();
   const Geo& g = a.g;
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(32 * W, quad_min_warps<Q>() / W)
   const uint32_t i1m = i1 == 0 ? g.n1 - 1 : i1 - 1, i1p = i1 + 1 == g.n1 ? 0u : i1 + 1;
   grid_wait_previous();
   const S* pin = static_cast<const S*>(a.pin);
-  float d[4][Q];
+  F2 d[2][Q];
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     const int c0 = Lat<Q>::c0(q), c1 = Lat<Q>::c1(q);
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(32 * W, quad_min_warps<Q>() / W)
 // the linear cell index and each lane finds its own row; the lanes past the
 // last quad redo it without storing.
 template <int Q, class S, bool FACES, bool FORCE>
-__global__ void __launch_bounds__(kBlock, quad_min_warps<Q>() / (kBlock / 32))
+__global__ void __launch_bounds__(kBlock, quad_min_warps<Q, FORCE>() / (kBlock / 32))
     k_step_gquad(const __grid_constant__ StepArgs a) {
   grid_launch_next();
   const Geo& g = a.g;
@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(kBlock, quad_min_warps<Q>() / (kBlock / 32))
   const uint32_t i1m = i1 == 0 ? g.n1 - 1 : i1 - 1, i1p = i1 + 1 == g.n1 ? 0u : i1 + 1;
   grid_wait_previous();
   const S* pin = static_cast<const S*>(a.pin);
-  float d[4][Q];
+  F2 d[2][Q];
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     const int c0 = Lat<Q>::c0(q), c1 = Lat<Q>::c1(q);
@@ -473,7 +473,7 @@ __device__ __forceinline__ void gpair_step(const StepArgs& a, uint32_t pidx) {
 }
 
 template <int Q, class S, bool FACES, bool FORCE>
-__global__ void __launch_bounds__(kBlock, kGPairMinWarps / (kBlock / 32))
+__global__ void __launch_bounds__(kBlock, kPairMinWarps / (kBlock / 32))
     k_step_gpair(const __grid_constant__ StepArgs a) {
   grid_launch_next();
   grid_wait_previous();
@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(kBlock, kGPairMinWarps / (kBlock / 32))
 // kBatchTile cells is kBatchTile / 2 pairs, kBatchTile / (2 kBlock) per thread
 // (see k_batched_step for the tile walk and SPEC).
 template <int Q, class S, int SPEC, bool PAD>
-__global__ void __launch_bounds__(kBlock, kGPairMinWarps / (kBlock / 32))
+__global__ void __launch_bounds__(kBlock, kPairMinWarps / (kBlock / 32))
     k_batched_pair(const StepArgs* __restrict__ args, const BatchTile* __restrict__ tiles,
                    uint32_t ntiles, int which) {
   grid_launch_next();

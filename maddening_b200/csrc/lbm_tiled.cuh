@@ -233,19 +233,6 @@ __device__ __forceinline__ void collide_ref(const StepArgs& a, uint32_t c, float
   }
 }
 
-// Wall-node swap of a lane's two cells (w0, w1: it is a wall cell).
-template <int Q>
-__device__ __forceinline__ void wall_swap2(F2 (&d)[Q], bool w0, bool w1) {
-#pragma unroll
-  for (int q = 1; q < Q; ++q) {
-    const int o = Lat<Q>::opp(q);
-    if (q > o) continue;
-    const F2 x = d[q], y = d[o];
-    d[q] = F2(w0 ? y.v.x : x.v.x, w1 ? y.v.y : x.v.y);
-    d[o] = F2(w0 ? x.v.x : y.v.x, w1 ? x.v.y : y.v.y);
-  }
-}
-
 // collide_ref for the two cells of a lane (c0, c1), two-wide arithmetic.
 template <int Q, class S, bool FORCE>
 __device__ __forceinline__ void collide_ref2(const StepArgs& a, uint32_t c0, uint32_t c1,
