@@ -60,6 +60,20 @@ bool fastdiv_ok(const lbm::FastDiv& f, uint32_t xmax) {
 
 
 
+// The geometry with state rows padded to n2 + 1 cells; false where a padded
+// state of Q planes does not index below 2^32.
+bool pad_rows(const lbm::Geo& g, int Q, lbm::Geo* out) {
+  *out = g;
+  const uint64_t rs = uint64_t(g.n2) + 1;
+  const uint64_t ps = uint64_t(g.n0) * g.n1 * rs;
+  if (ps * Q >= (uint64_t(1) << 32)) return false;
+  out->rstride = static_cast<uint32_t>(rs);
+  out->splane = static_cast<uint32_t>(uint64_t(g.n1) * rs);
+  out->pstride = static_cast<uint32_t>(ps);
+  out->div_rstride = make_fastdiv(out->rstride);
+  return fastdiv_ok(out->div_rstride, static_cast<uint32_t>(ps));
+}
+
 // Maps one face condition of the ABI to the kernel form (internal axes).
 int map_face(const lbm_plan* p, const lbm_face_bc& in, bool is_outlet, lbm::FaceK* out) {
   std::memset(out, 0, sizeof(*out));
@@ -133,12 +147,12 @@ int build_args(const lbm_plan* p, const lbm_step_args* args, const lbm_moments* 
 
 template <int Q>
 int dispatch_s(const lbm_plan* p, cudaStream_t s, const lbm::StepArgs& a, const void* f_in,
-               void* f_out, int64_t n, char* ws) {
+               void* f_out, int64_t n, char* ws, size_t wb) {
   switch (p->storage) {
-    case LBM_STORE_F32: return run_steps<Q, float>(p, s, a, f_in, f_out, n, ws);
-    case LBM_STORE_F16: return run_steps<Q, __half>(p, s, a, f_in, f_out, n, ws);
-    case LBM_STORE_BF16: return run_steps<Q, __nv_bfloat16>(p, s, a, f_in, f_out, n, ws);
-    case LBM_STORE_F64: return run_steps<Q, double>(p, s, a, f_in, f_out, n, ws);
+    case LBM_STORE_F32: return run_steps<Q, float>(p, s, a, f_in, f_out, n, ws, wb);
+    case LBM_STORE_F16: return run_steps<Q, __half>(p, s, a, f_in, f_out, n, ws, wb);
+    case LBM_STORE_BF16: return run_steps<Q, __nv_bfloat16>(p, s, a, f_in, f_out, n, ws, wb);
+    case LBM_STORE_F64: return run_steps<Q, double>(p, s, a, f_in, f_out, n, ws, wb);
   }
   return fail(LBM_ERR_INVALID, "bad storage");
 }
@@ -158,8 +172,8 @@ int do_steps(const lbm_plan* p, lbm_stream_t stream, const void* f_in, void* f_o
   if (rc) return rc;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(workspace);
-  return p->Q == 19 ? dispatch_s<19>(p, s, a, f_in, f_out, n, ws)
-                    : dispatch_s<9>(p, s, a, f_in, f_out, n, ws);
+  return p->Q == 19 ? dispatch_s<19>(p, s, a, f_in, f_out, n, ws, workspace_bytes)
+                    : dispatch_s<9>(p, s, a, f_in, f_out, n, ws, workspace_bytes);
 }
 
 
@@ -340,6 +354,7 @@ int lbm_plan_create(const lbm_desc* desc, lbm_plan** plan) {
     delete p;
     return fail(LBM_ERR_INVALID, "internal: index division constants failed self-check");
   }
+  p->gpad_ok = pad_rows(p->g, p->Q, &p->gpad);
   *plan = p;
   return LBM_OK;
 }
@@ -357,7 +372,7 @@ int lbm_state_bytes(const lbm_plan* plan, size_t* bytes) {
 
 int lbm_workspace_bytes(const lbm_plan* plan, size_t* bytes) {
   if (plan == nullptr || bytes == nullptr) return fail(LBM_ERR_INVALID, "NULL argument");
-  *bytes = 2 * align256(state_bytes(plan)) + 256;
+  *bytes = rollout_bytes(plan);
   return LBM_OK;
 }
 
@@ -739,17 +754,9 @@ int lbm_batch_create(const lbm_plan* const* plans, int32_t n, lbm_batch** out) {
     b->plans.push_back(p);
     // A paired member with odd rows keeps its state rows padded to n2 + 1.
     lbm::Geo g = p->g;
-    if (pairable(i) && g.n2 % 2 == 1) {
-      const uint64_t rs = uint64_t(g.n2) + 1;
-      const uint64_t ps = uint64_t(g.n0) * g.n1 * rs;
-      g.rstride = static_cast<uint32_t>(rs);
-      g.splane = static_cast<uint32_t>(uint64_t(g.n1) * rs);
-      g.div_rstride = make_fastdiv(g.rstride);
-      if (ps * p->Q >= (uint64_t(1) << 32) || !fastdiv_ok(g.div_rstride, static_cast<uint32_t>(ps))) {
-        delete b;
-        return fail(LBM_ERR_INVALID, "instance %d: padded rows exceed 32-bit indexing", i);
-      }
-      g.pstride = static_cast<uint32_t>(ps);
+    if (pairable(i) && g.n2 % 2 == 1 && !pad_rows(p->g, p->Q, &g)) {
+      delete b;
+      return fail(LBM_ERR_INVALID, "instance %d: padded rows exceed 32-bit indexing", i);
     }
     b->sgeo.push_back(g);
     for (uint32_t c = 0; c < g.ncell; c += lbm::kBatchTile)

@@ -22,6 +22,13 @@ struct lbm_plan {
   size_t elem = 4;               // bytes per stored population
   size_t io = 4;                 // bytes per f / force / moment element
   uint32_t flags = 0;            // LBM_PLAN_* bits
+  lbm::Geo gpad{};               // the geometry with state rows of n2 + 1 cells
+  bool gpad_ok = false;          // ... indexes below 2^32
+
+  // 16-bit states with odd rows are kept padded inside a rollout.
+  bool odd_rows_padded() const {
+    return elem == 2 && g.n2 % 2 == 1 && gpad_ok && !(flags & LBM_PLAN_SINGLE_CELLS);
+  }
 };
 
 // Records the message for lbm_last_error (calling thread) and returns code.
@@ -33,6 +40,15 @@ inline size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 
 inline size_t state_bytes(const lbm_plan* p) {
   return static_cast<size_t>(p->Q) * static_cast<size_t>(p->g.ncell) * p->elem;
+}
+
+inline size_t padded_state_bytes(const lbm_plan* p) {
+  return static_cast<size_t>(p->Q) * static_cast<size_t>(p->gpad.pstride) * p->elem;
+}
+// Workspace of a rollout of more than one step: two state copies, a status word.
+inline size_t rollout_bytes(const lbm_plan* p) {
+  const size_t sb = p->odd_rows_padded() ? padded_state_bytes(p) : state_bytes(p);
+  return 2 * align256(sb) + 256;
 }
 
 inline unsigned grid_for(uint64_t n) { return static_cast<unsigned>((n + lbm::kBlock - 1) / lbm::kBlock); }
@@ -69,7 +85,7 @@ int run_padded(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f
                char* ws);
 template <int Q, class S>
 int run_steps(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in, void* f_out,
-              int64_t n, char* ws);
+              int64_t n, char* ws, size_t ws_bytes);
 template <int Q, class S>
 int run_history(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in,
                 void* f_out, int64_t n, int64_t every, const lbm_history* h, char* ws);

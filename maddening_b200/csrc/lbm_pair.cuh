@@ -25,8 +25,9 @@
 // like the scalar one, so the results are bit-identical; the wall swap is skipped by warps without a wall cell and the
 // face checks by pairs that cannot touch a face.
 //
-// A second form (k_step_gpair) takes any even row length: pairs follow the
-// instance-wide cell index and each lane finds its own row.
+// A second form (k_step_gpair) takes any row length: pairs follow the
+// instance-wide cell index and each lane finds its own row.  Odd rows are kept
+// padded to n2 + 1 in the state planes (PAD).
 //
 // Requirements (checked on the host): an even contiguous extent n2 (a multiple
 // of 64 W for the row-segment form), state planes and the wall mask aligned for
@@ -472,12 +473,12 @@ __device__ __forceinline__ void gpair_step(const StepArgs& a, uint32_t pidx) {
   pair_finish<Q, S, FACES, FORCE, PAD>(a, i0, i1, k, r * g.n2, srow, v, e, valid);
 }
 
-template <int Q, class S, bool FACES, bool FORCE>
+template <int Q, class S, bool FACES, bool FORCE, bool PAD>
 __global__ void __launch_bounds__(kBlock, kPairMinWarps / (kBlock / 32))
     k_step_gpair(const __grid_constant__ StepArgs a) {
   grid_launch_next();
   grid_wait_previous();
-  gpair_step<Q, S, FACES, FORCE, false>(a, blockIdx.x * kBlock + threadIdx.x);
+  gpair_step<Q, S, FACES, FORCE, PAD>(a, blockIdx.x * kBlock + threadIdx.x);
 }
 
 // Batched ensemble, state steps of members with even rows: a tile of
