@@ -147,3 +147,30 @@ int run_pipe_mp(const lbm_plan* p, cudaStream_t s, const lbm::StepArgs& a,
 // rollout).  Instantiated for Q in {9, 19}, S in {float, __half, __nv_bfloat16}.
 template <int Q, class S, int MODE>
 int launch_tiled(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s);
+
+// The fluid half of one pipe-node step (force mode 3) in one pass: f_bc and the
+// moments (D3Q19 FP32).
+template <int Q, class S>
+int launch_tiled_pipe(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s);
+
+// Whether the one-pass step can take the call: 32-bit IO, rows of a multiple of
+// 4 cells (16-byte copy units), 16-byte aligned reference-layout buffers that do
+// not overlap, an unpadded whole lattice; status: where its status word goes.
+template <class S>
+bool tiled_ok(const lbm_plan* p, const lbm::StepArgs& a, const void* status, bool aos_out) {
+  if constexpr (sizeof(typename lbm::StoreT<S>::IO) != 4) {
+    return false;
+  } else {
+    if (p->flags & LBM_PLAN_TWO_PASS) return false;
+    if (p->g.n2 % 4 != 0 || a.g.rstride != a.g.n2 || a.face_inset != 0) return false;
+    const uintptr_t fi = reinterpret_cast<uintptr_t>(a.f_in);
+    const uintptr_t fo = reinterpret_cast<uintptr_t>(a.f_out);
+    if (fi % 16 != 0) return false;
+    if (aos_out) {
+      // f_out is written while other blocks still read f_in: no overlap
+      const uintptr_t bytes = static_cast<uintptr_t>(p->g.ncell) * p->Q * 4;
+      if (fo % 16 != 0 || (fo < fi + bytes && fi < fo + bytes)) return false;
+    }
+    return reinterpret_cast<uintptr_t>(status) % 4 == 0;
+  }
+}

@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <type_traits>
 #include <utility>
 
 #include "lbm_host.h"
@@ -10,7 +11,10 @@
 
 // Single-phase pipe rollout: one fused launch per step (k_pipe_step: D3Q19
 // pull step + the tracer of the same cell), tracer populations ping-ponged
-// between two plane sets.
+// between two plane sets.  A single step (the call a graph manager makes) runs
+// its fluid half in one pass over the reference layout instead, then the
+// tracer with the velocity that pass wrote: 173 + 69 + 60 B per cell for 496
+// (256 x 128 x 128 FP32: 351 -> 271 us).
 template <class S>
 int run_pipe(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_in, void* f_out,
              const void* t_in, void* t_out, int64_t n, double tau_tracer, void* tracer_out,
@@ -28,37 +32,54 @@ int run_pipe(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_i
   t.inv_tau = 1.0 / tau_tracer;
   t.f7_in = t_in;
   t.tout = T[0];
-  lbm::k_tracer_prepare<IO><<<grid, lbm::kBlock, 0, s>>>(t);
-  int rc = cuda_check(cudaGetLastError(), "k_tracer_prepare launch");
-  if (rc) return rc;
-  lbm::StepArgs m = a;
-  m.rho = m.prs = m.vel = nullptr;
-  m.f_in = f_in;
-  m.pout = A;
-  rc = launch_prepare<19, S>(m, s);
-  if (rc) return rc;
-  int cur = 0;
-  for (int64_t i = 1; i < n; ++i) {
-    m.pin = A;
-    m.pout = B;
-    t.tin = T[cur];
-    t.tout = T[1 - cur];
-    launch_after(lbm::k_pipe_step<S, false>, grid, lbm::kBlock, s, m, t);
-    rc = cuda_check(cudaGetLastError(), "k_pipe_step launch");
-    if (rc) return rc;
-    cur = 1 - cur;
-    std::swap(A, B);
-  }
-  a.pin = A;
+  a.f_in = f_in;
   a.f_out = f_out;
   a.prs = nullptr;
-  a.mflags &= ~lbm::kMomRawVelocity;
-  t.tin = T[cur];
-  t.tout = T[1 - cur];
-  launch_after(lbm::k_pipe_step<S, true>, grid, lbm::kBlock, s, a, t);
-  rc = cuda_check(cudaGetLastError(), "k_pipe_step launch");
-  if (rc) return rc;
-  cur = 1 - cur;
+  int rc;
+  bool done = false;
+  if constexpr (std::is_same<S, float>::value) {
+    if (n == 1 && tiled_ok<S>(p, a, ws, true)) {
+      lbm::StepArgs m = a;
+      m.mflags &= ~lbm::kMomRawVelocity;
+      if (m.vel == nullptr) m.vel = ws + 2 * sb + 2 * tb;
+      m.status = reinterpret_cast<int*>(ws);
+      rc = cuda_check(cudaMemsetAsync(m.status, 0, sizeof(int), s), "cudaMemsetAsync");
+      if (rc) return rc;
+      rc = launch_tiled_pipe<19, S>(p, m, s);
+      if (rc) return rc;
+      t.vel = m.vel;
+      lbm::k_tracer_step<IO><<<grid, lbm::kBlock, 0, s>>>(t);
+      rc = cuda_check(cudaGetLastError(), "k_tracer_step launch");
+      if (rc) return rc;
+      done = true;
+    }
+  }
+  int cur = 0;
+  if (!done) {
+    lbm::StepArgs m = a;
+    m.rho = m.vel = nullptr;
+    m.pout = A;
+    rc = launch_prepare<19, S>(m, s);
+    if (rc) return rc;
+    for (int64_t i = 1; i < n; ++i) {
+      m.pin = A;
+      m.pout = B;
+      if (i == 1) launch_after(lbm::k_pipe_step<S, true, false>, grid, lbm::kBlock, s, m, t);
+      else launch_after(lbm::k_pipe_step<S, false, false>, grid, lbm::kBlock, s, m, t);
+      rc = cuda_check(cudaGetLastError(), "k_pipe_step launch");
+      if (rc) return rc;
+      std::swap(A, B);
+      t.tin = T[cur];
+      cur = 1 - cur;
+      t.tout = T[cur];
+    }
+    a.pin = A;
+    a.mflags &= ~lbm::kMomRawVelocity;
+    if (n == 1) launch_after(lbm::k_pipe_step<S, true, true>, grid, lbm::kBlock, s, a, t);
+    else launch_after(lbm::k_pipe_step<S, false, true>, grid, lbm::kBlock, s, a, t);
+    rc = cuda_check(cudaGetLastError(), "k_pipe_step launch");
+    if (rc) return rc;
+  }
   t.tin = T[cur];
   t.f7_out = t_out;
   t.tracer_out = tracer_out;

@@ -32,30 +32,24 @@ struct TracerArgs {
   const void* tin;      // populations (7 planes)
   void* tout;
   double inv_tau;       // 1 / tau_tracer
-  const void* f7_in;    // (grid, 7) reference layout (prepare)
+  const void* f7_in;    // (grid, 7) reference layout (first step)
+  const void* vel;      // (grid, 3) velocity of this step (k_tracer_step)
   void* f7_out;         // (grid, 7) reference layout (final)
   void* tracer_out;     // grid (final)
 };
 
-template <class IO>
-__global__ void __launch_bounds__(kBlock) k_tracer_prepare(const TracerArgs a) {
-  const uint32_t c = blockIdx.x * kBlock + threadIdx.x;
-  const IO* fi = aos_fill<7, IO>(static_cast<const IO*>(a.f7_in), blockIdx.x * kBlock, a.g.ncell);
-  if (c >= a.g.ncell) return;
-#pragma unroll
-  for (int q = 0; q < 7; ++q) static_cast<IO*>(a.tout)[static_cast<size_t>(q) * a.g.ncell + c] = fi[q];
-}
-
-// Tracer step of cell x with this step's velocity uu (0 in walls).
+// Tracer step of cell x with this step's velocity uu (0 in walls).  row: the
+// cell's populations in the reference layout (a tile row), or NULL: the planes.
 template <class IO>
 __device__ __forceinline__ void tracer_cell(const TracerArgs& a, const Cell& x, bool wall,
-                                            const IO (&uu)[3]) {
+                                            const IO (&uu)[3], const IO* row = nullptr) {
   const Geo& g = a.g;
   const uint32_t c = x.c;
   const IO* tin = static_cast<const IO*>(a.tin);
   IO t[7];
 #pragma unroll
-  for (int q = 0; q < 7; ++q) t[q] = tin[static_cast<size_t>(q) * g.ncell + c];
+  for (int q = 0; q < 7; ++q)
+    t[q] = row != nullptr ? row[q] : tin[static_cast<size_t>(q) * g.ncell + c];
   if (!wall) {
     IO tracer = t[0];
 #pragma unroll
@@ -86,10 +80,10 @@ __device__ __forceinline__ void tracer_cell(const TracerArgs& a, const Cell& x, 
 
 // One pipe-node step of cell x: the D3Q19 pull step with the pipe force
 // (force mode 3: no half-force step in the moments), then the tracer step of
-// the same cell with the velocity just taken (lbm_pipe.py:751-879).  LAST
-// writes f_bc in the reference layout and the moment outputs instead of
-// colliding.
-template <class S, bool LAST>
+// the same cell with the velocity just taken (lbm_pipe.py:751-879).  FIRST reads
+// the tracer in the reference layout; LAST writes f_bc in the reference layout
+// and the moment outputs instead of colliding.
+template <class S, bool FIRST, bool LAST>
 __global__ void __launch_bounds__(kBlock, min_blocks<S>())
     k_pipe_step(const __grid_constant__ StepArgs a, const __grid_constant__ TracerArgs t) {
   using R = typename StoreT<S>::R;
@@ -97,6 +91,9 @@ __global__ void __launch_bounds__(kBlock, min_blocks<S>())
   grid_launch_next();
   const uint32_t cidx = blockIdx.x * kBlock + threadIdx.x;
   grid_wait_previous();
+  const IO* trow = nullptr;
+  if constexpr (FIRST)
+    trow = aos_fill<7, IO>(static_cast<const IO*>(t.f7_in), blockIdx.x * kBlock, a.g.ncell);
   if (cidx < a.g.ncell) {
     const Cell x = locate(a.g, cidx);
     R d[19];
@@ -121,9 +118,22 @@ __global__ void __launch_bounds__(kBlock, min_blocks<S>())
     const IO uu[3] = {wall ? IO(0) : static_cast<IO>(m.u[0]),
                       wall ? IO(0) : static_cast<IO>(m.u[1]),
                       wall ? IO(0) : static_cast<IO>(m.u[2])};
-    tracer_cell<IO>(t, x, wall, uu);
+    tracer_cell<IO>(t, x, wall, uu, trow);
   }
   if (LAST) aos_flush<19, IO>(static_cast<IO*>(a.f_out), blockIdx.x * kBlock, a.g.ncell);
+}
+
+// Tracer step of a single update whose fluid half ran in one pass: reference
+// layout in, the new velocity (0 in walls) from memory, pushed into the planes.
+template <class IO>
+__global__ void __launch_bounds__(kBlock) k_tracer_step(const __grid_constant__ TracerArgs t) {
+  const uint32_t cidx = blockIdx.x * kBlock + threadIdx.x;
+  const IO* row = aos_fill<7, IO>(static_cast<const IO*>(t.f7_in), blockIdx.x * kBlock, t.g.ncell);
+  if (cidx >= t.g.ncell) return;
+  const Cell x = locate(t.g, cidx);
+  const IO* v = static_cast<const IO*>(t.vel) + static_cast<size_t>(cidx) * 3;
+  const IO uu[3] = {v[0], v[1], v[2]};
+  tracer_cell<IO>(t, x, t.wall != nullptr && t.wall[cidx] != 0, uu, row);
 }
 
 // Last pass: populations to the reference layout and the tracer field.

@@ -172,30 +172,6 @@ int launch_step_padded(const lbm::StepArgs& a, cudaStream_t s) {
   return cuda_check(cudaGetLastError(), "k_step_padded launch");
 }
 
-// One-pass tiled step (lbm_tiled.cuh) for lbm_update and the first step of a
-// rollout: 32-bit IO, rows of a multiple of 4 cells (16-byte copy groups),
-// 16-byte aligned reference-layout buffers that do not overlap, an unpadded
-// whole lattice.
-template <class S>
-bool tiled_ok(const lbm_plan* p, const lbm::StepArgs& a, const void* ws, bool aos_out) {
-  if constexpr (sizeof(typename lbm::StoreT<S>::IO) != 4) {
-    return false;
-  } else {
-    if (p->flags & LBM_PLAN_TWO_PASS) return false;
-    if (p->g.n2 % 4 != 0 || p->g.rstride != p->g.n2 || a.face_inset != 0 || a.force_mode == 3)
-      return false;
-    const uintptr_t fi = reinterpret_cast<uintptr_t>(a.f_in);
-    const uintptr_t fo = reinterpret_cast<uintptr_t>(a.f_out);
-    if (fi % 16 != 0) return false;
-    if (aos_out) {
-      // f_out is written while other blocks still read f_in: no overlap
-      const uintptr_t bytes = static_cast<uintptr_t>(p->g.ncell) * p->Q * 4;
-      if (fo % 16 != 0 || (fo < fi + bytes && fi < fo + bytes)) return false;
-    }
-    return reinterpret_cast<uintptr_t>(ws) % 4 == 0;  // the status word
-  }
-}
-
 }  // namespace
 
 template <int Q, class S>

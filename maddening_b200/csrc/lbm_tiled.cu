@@ -1,6 +1,7 @@
 // Launchers of the one-pass tiled step (lbm_tiled.cuh), in a translation unit
 // of their own so that the library's units compile in parallel.
 #include <algorithm>
+#include <type_traits>
 
 #include "lbm_host.h"
 #include "lbm_tiled.cuh"
@@ -41,9 +42,9 @@ lbm::TileGeo tile_geo(const lbm_plan* p, uint32_t grid) {
   return t;
 }
 
-template <int Q, class S, int MODE, bool FACES, bool FORCE>
+template <int Q, class S, int MODE, bool FACES, bool FORCE, bool PIPE = false>
 int launch_tiled_t(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s) {
-  auto kern = lbm::k_tiled<Q, S, MODE, FACES, FORCE>;
+  auto kern = lbm::k_tiled<Q, S, MODE, FACES, FORCE, PIPE>;
   constexpr size_t smem = lbm::tiled_smem_bytes<Q, MODE>();
   int rc = cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            static_cast<int>(smem)),
@@ -78,9 +79,18 @@ int launch_tiled(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s) {
                : launch_tiled_t<Q, S, MODE, false, false>(p, a, s);
 }
 
+template <int Q, class S>
+int launch_tiled_pipe(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s) {
+  if constexpr (Q == 19 && std::is_same<S, float>::value)
+    return launch_tiled_t<Q, S, lbm::kOutAoS, false, false, true>(p, a, s);
+  else
+    return fail(LBM_ERR_UNSUPPORTED, "the one-pass pipe step is D3Q19 FP32");
+}
+
 #define LBM_TILED_INST(Q, S)                                                             \
   template int launch_tiled<Q, S, lbm::kOutAoS>(const lbm_plan*, const lbm::StepArgs&,   \
                                                 cudaStream_t);                           \
   template int launch_tiled<Q, S, lbm::kOutState>(const lbm_plan*, const lbm::StepArgs&, \
-                                                  cudaStream_t);
+                                                  cudaStream_t);                          \
+  template int launch_tiled_pipe<Q, S>(const lbm_plan*, const lbm::StepArgs&, cudaStream_t);
 LBM_TILED_INST(LBM_UNIT_Q, LBM_UNIT_S)

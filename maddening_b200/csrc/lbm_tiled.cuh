@@ -37,8 +37,7 @@
 //
 // Requirements (checked on the host): 32-bit IO (FP32, FP16 or BF16
 // storage), an a2 extent that is a multiple of 4, f_in (and f_out for
-// kOutAoS) 16-byte aligned and not overlapping, no halo-padded block, no
-// pipe force.  Every wait is bounded in time and also ends when another warp
+// kOutAoS) 16-byte aligned and not overlapping, no halo-padded block.  Every wait is bounded in time and also ends when another warp
 // has given up; then the block sets bit 0 of *status, waits (bounded) for its
 // own copies in flight and returns.
 #pragma once
@@ -265,6 +264,22 @@ __device__ __forceinline__ void collide_ref2(const StepArgs& a, uint32_t c0, uin
   }
 }
 
+// The pipe node's collide of a lane's two cells (k_prepare's with force mode 3):
+// no half-force step in the moments; w0, w1: wall cells.  i0: the cells' plane.
+__device__ __forceinline__ void collide_pipe2(const StepArgs& a, uint32_t i0, uint32_t c0,
+                                              uint32_t c1, bool w0, bool w1, F2 (&d)[19]) {
+  float f0 = 0, f1 = 0;
+  if (i0 == a.prop_x) {
+    const uint32_t base = i0 * a.g.plane;
+    if (__ldg(a.prop_mask + (c0 - base)) != 0) f0 = static_cast<float>(a.force[0]);
+    if (__ldg(a.prop_mask + (c1 - base)) != 0) f1 = static_cast<float>(a.force[0]);
+  }
+  const float gz = static_cast<float>(a.force[2]);
+  const F2 F[3] = {F2(f0, f1), F2(0.0f), F2(w0 ? 0.0f : gz, w1 ? 0.0f : gz)};
+  const Mom<F2> m = moments<19, F2, true>(d, F, false);
+  collide<19, F2, true>(d, m, F, F2(a.omega), F2(a.guo_c));
+}
+
 // Population qs of p = C(f) at cell c, from the reference state in global
 // memory (zero-gradient faces reach cells outside the buffered planes).
 template <int Q, class S, bool FORCE>
@@ -404,12 +419,15 @@ struct Ring {
   }
 };
 
-template <int Q, class S, int MODE, bool FACES, bool FORCE>
+// PIPE: the pipe node's force (force mode 3), f_bc and moments out, no faces.
+template <int Q, class S, int MODE, bool FACES, bool FORCE, bool PIPE = false>
 __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
     k_tiled(const __grid_constant__ StepArgs a, const __grid_constant__ TileGeo t) {
   using T = TileShape<Q>;
   using R = float;
   static_assert(MODE == kOutAoS || MODE == kOutState, "f_bc out or the next state out");
+  static_assert(!PIPE || (Q == 19 && sizeof(S) == 4 && MODE == kOutAoS && !FACES && !FORCE),
+                "the pipe node's update");
   constexpr uint32_t S_ = Sweep<Q>::SLOTS;
   static_assert(Sweep<Q>::SLOTS >= 5, "ring depth: three planes read, one collided, one landing");
   extern __shared__ __align__(128) unsigned char smem[];
@@ -496,7 +514,10 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
       for (int q = 0; q < Q; ++q) d[q] = F2(slot[soff[0] + q], slot[soff[1] + q]);
 #pragma unroll
       for (int q = 0; q < Q; ++q) d[q] = to_offset<Q, F2>(d[q], q);
-      collide_ref2<Q, S, FORCE>(a, cs0 + rz[0], cs0 + rz[1], d);
+      if constexpr (PIPE)
+        collide_pipe2(a, plane_s(t, C), cs0 + rz[0], cs0 + rz[1], wb[0] != 0, wb[1] != 0, d);
+      else
+        collide_ref2<Q, S, FORCE>(a, cs0 + rz[0], cs0 + rz[1], d);
       __syncwarp();
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
