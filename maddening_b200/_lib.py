@@ -11,6 +11,8 @@ import os
 import threading
 from pathlib import Path
 
+import torch
+
 _PKG = Path(__file__).resolve().parent
 LIB_PATH = _PKG / "liblbm_b200.so"
 
@@ -132,6 +134,21 @@ def last_error() -> str:
     return buf.value.decode(errors="replace")
 
 
+def tensor_on(x, dev):
+    """``torch.as_tensor(x, device=dev)``, without the call for a tensor that is
+    there already (a step of a small lattice is bound by such calls)."""
+    if type(x) is torch.Tensor and x.device == dev:
+        return x
+    return torch.as_tensor(x, device=dev)
+
+
+def raw_stream(dev) -> int:
+    """Handle of the current stream of ``dev``."""
+    index = dev.index
+    return torch._C._cuda_getCurrentRawStream(
+        torch.cuda.current_device() if index is None else index)
+
+
 def check(status: int) -> None:
     if status != LBM_OK:
         raise LbmError(status, last_error())
@@ -151,6 +168,7 @@ class Plan:
         h = _P()
         check(lib().lbm_plan_create(C.byref(d), C.byref(h)))
         self._h = h
+        self._sizes = {}
         self.q = q
         self.shape = tuple(int(n) for n in shape)
         self.tau = float(tau)
@@ -162,9 +180,13 @@ class Plan:
         return self._h
 
     def _size(self, fn) -> int:
-        n = C.c_size_t()
-        check(fn(self._h, C.byref(n)))
-        return int(n.value)
+        """A size that depends on the plan alone, asked for once."""
+        name = fn.__name__
+        if name not in self._sizes:
+            n = C.c_size_t()
+            check(fn(self._h, C.byref(n)))
+            self._sizes[name] = int(n.value)
+        return self._sizes[name]
 
     def state_bytes(self) -> int:
         return self._size(lib().lbm_state_bytes)

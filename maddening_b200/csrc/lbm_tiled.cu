@@ -1,6 +1,7 @@
 // Launchers of the one-pass tiled step (lbm_tiled.cuh), in a translation unit
 // of their own so that the library's units compile in parallel.
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "lbm_host.h"
@@ -56,10 +57,17 @@ int launch_tiled_t(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s) {
   rc = cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev),
                   "cudaDeviceGetAttribute");
   if (rc) return rc;
-  rc = cuda_check(
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, lbm::TileShape<Q>::NT, smem),
-      "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-  if (rc) return rc;
+  // blocks per SM of this kernel: the same on every call and every device (the
+  // library is built for one architecture), so the occupancy query runs once
+  static std::atomic<int> blocks{0};
+  per_sm = blocks.load(std::memory_order_relaxed);
+  if (per_sm == 0) {
+    rc = cuda_check(
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, lbm::TileShape<Q>::NT, smem),
+        "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+    if (rc) return rc;
+    if (per_sm > 0) blocks.store(per_sm, std::memory_order_relaxed);
+  }
   if (per_sm < 1) return fail(LBM_ERR_CUDA, "tiled step: no resident block (%zu B smem)", smem);
   const uint32_t grid = static_cast<uint32_t>(per_sm) * static_cast<uint32_t>(sms);
   const lbm::TileGeo t = tile_geo<Q>(p, grid);

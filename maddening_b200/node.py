@@ -54,6 +54,8 @@ def prescribed_density(pressure, cs2: float = 1.0 / 3.0):
     float64 or Python input in float64.  Returns a Python float for host
     inputs and a 0-d CUDA tensor for device inputs.
     """
+    if type(pressure) is float:
+        return pressure / cs2
     if isinstance(pressure, torch.Tensor):
         if pressure.is_cuda:
             return pressure.reshape(()) / cs2
@@ -133,6 +135,7 @@ class LBMNode(SimulationNode):
         self._storage = storage
         self._io_dtype = torch.float64 if storage == "f64" else torch.float32
         self._device = torch.device(device) if device is not None else None
+        self._dev_ready = False
         if wall_mask is not None:
             wall_mask = np.asarray(wall_mask)
             if wall_mask.shape != self._grid_shape:
@@ -186,10 +189,12 @@ class LBMNode(SimulationNode):
         return bool(self.halo_width())
 
     def _dev(self) -> torch.device:
-        if not torch.cuda.is_available():
-            raise RuntimeError("LBMNode needs a CUDA device (sm_100a); there is no CPU path")
-        if self._device is None:
-            self._device = torch.device("cuda", torch.cuda.current_device())
+        if not self._dev_ready:  # asked once: a CUDA device does not go away
+            if not torch.cuda.is_available():
+                raise RuntimeError("LBMNode needs a CUDA device (sm_100a); there is no CPU path")
+            if self._device is None:
+                self._device = torch.device("cuda", torch.cuda.current_device())
+            self._dev_ready = True
         return self._device
 
     def _wall_mask_on(self, dev) -> torch.Tensor:
@@ -215,7 +220,7 @@ class LBMNode(SimulationNode):
         f = torch.empty(self._grid_shape + (self._Q,), dtype=self._io_dtype, device=dev)
         rho = None if density is None else self._as_field(density, self._grid_shape, dev)
         u = None if velocity is None else self._as_field(velocity, self._grid_shape + (self._D,), dev)
-        stream = torch.cuda.current_stream(dev).cuda_stream
+        stream = _lib.raw_stream(dev)
         _lib.check(_lib.lib().lbm_equilibrium(
             self._plan.handle, stream, None if rho is None else rho.data_ptr(),
             None if u is None else u.data_ptr(), f.data_ptr()))
@@ -241,9 +246,9 @@ class LBMNode(SimulationNode):
         shape = self._grid_shape if shape is None else tuple(shape)
         # wall mask precedence: wall_mask_update > state["wall_mask"] > node mask
         if "wall_mask_update" in bi:
-            wall = torch.as_tensor(bi["wall_mask_update"], device=dev)
+            wall = _lib.tensor_on(bi["wall_mask_update"], dev)
         elif "wall_mask" in state:
-            wall = torch.as_tensor(state["wall_mask"], device=dev)
+            wall = _lib.tensor_on(state["wall_mask"], dev)
         else:
             wall = self._wall_mask_on(dev)
         if tuple(wall.shape) != shape:
@@ -334,16 +339,15 @@ class LBMNode(SimulationNode):
     def _outputs(self, dev):
         shape = self._grid_shape
         f = torch.empty(shape + (self._Q,), dtype=self._io_dtype, device=dev)
-        rho = torch.empty(shape, dtype=self._io_dtype, device=dev)
-        vel = torch.empty(shape + (self._D,), dtype=self._io_dtype, device=dev)
-        prs = torch.empty(shape, dtype=self._io_dtype, device=dev)
+        rho = f.new_empty(shape)
+        vel = f.new_empty(shape + (self._D,))
+        prs = f.new_empty(shape)
         m = _lib.lbm_moments()
         m.density, m.velocity, m.pressure = rho.data_ptr(), vel.data_ptr(), prs.data_ptr()
         return f, rho, vel, prs, m
 
     def _f_in(self, state, dev) -> torch.Tensor:
-        f = state["f"]
-        f = torch.as_tensor(f, device=dev)
+        f = _lib.tensor_on(state["f"], dev)
         if f.dtype != self._io_dtype:
             f = f.to(self._io_dtype)
         if tuple(f.shape) != self._grid_shape + (self._Q,):
@@ -358,7 +362,7 @@ class LBMNode(SimulationNode):
         f, rho, vel, prs, m = self._outputs(dev)
         nbytes = self._plan.workspace_bytes() if n_steps > 1 else self._plan.state_bytes()
         ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-        stream = torch.cuda.current_stream(dev).cuda_stream
+        stream = _lib.raw_stream(dev)
         lib = _lib.lib()
         if n_steps == 1:
             rc = lib.lbm_update(self._plan.handle, stream, f_in.data_ptr(), f.data_ptr(),
@@ -406,7 +410,7 @@ class LBMNode(SimulationNode):
         for k, t in history.items():
             setattr(h, k, t.data_ptr() if nrec > 0 else None)
         ws = torch.empty(self._plan.workspace_bytes(), dtype=torch.uint8, device=dev)
-        stream = torch.cuda.current_stream(dev).cuda_stream
+        stream = _lib.raw_stream(dev)
         _lib.check(_lib.lib().lbm_rollout_history(
             self._plan.handle, stream, f_in.data_ptr(), f.data_ptr(), n, every, C.byref(args),
             C.byref(m), C.byref(h), ws.data_ptr(), ws.numel()))
@@ -476,7 +480,7 @@ class LBMNode(SimulationNode):
         m = _lib.lbm_moments()
         m.density, m.velocity, m.pressure = rho.data_ptr(), vel.data_ptr(), prs.data_ptr()
         ws = torch.empty(plan.state_bytes(), dtype=torch.uint8, device=dev)
-        stream = torch.cuda.current_stream(dev).cuda_stream
+        stream = _lib.raw_stream(dev)
         _lib.check(_lib.lib().lbm_update_padded(plan.handle, stream, f.data_ptr(),
                                                 f_out.data_ptr(), C.byref(args), C.byref(m),
                                                 ws.data_ptr(), ws.numel()))
@@ -563,7 +567,7 @@ class LBMNode(SimulationNode):
         f = self._f_in({"f": f}, dev)
         out = torch.empty(4, dtype=torch.float64, device=dev)
         ws = torch.empty(self._plan.reduce_workspace_bytes(), dtype=torch.uint8, device=dev)
-        stream = torch.cuda.current_stream(dev).cuda_stream
+        stream = _lib.raw_stream(dev)
         _lib.check(_lib.lib().lbm_mass_momentum(self._plan.handle, stream, f.data_ptr(),
                                                 out.data_ptr(), ws.data_ptr(), ws.numel()))
         return out[: 1 + self._D]
@@ -593,7 +597,7 @@ class _RolloutFn(torch.autograd.Function):
         f_out, rho, vel, prs, mom = node._outputs(dev)
         ws = torch.empty(plan.adjoint_workspace_bytes(n_steps, checkpoint_every),
                          dtype=torch.uint8, device=dev)
-        stream = torch.cuda.current_stream(dev).cuda_stream
+        stream = _lib.raw_stream(dev)
         _lib.check(_lib.lib().lbm_rollout_forward(
             plan.handle, stream, f_in.data_ptr(), f_out.data_ptr(), n_steps, checkpoint_every,
             C.byref(args), C.byref(mom), ws.data_ptr(), ws.numel()))
@@ -626,7 +630,7 @@ class _RolloutFn(torch.autograd.Function):
             n = node._D if len(ctx.force_shape) == 1 else int(np.prod(ctx.force_shape))
             gF = torch.empty(n, dtype=torch.float64, device=dev)
         gf0 = torch.empty_like(f_in) if want_f0 else None
-        stream = torch.cuda.current_stream(dev).cuda_stream
+        stream = _lib.raw_stream(dev)
         _lib.check(_lib.lib().lbm_rollout_backward(
             node.plan.handle, stream, f_in.data_ptr(), ctx.n_steps, ctx.K, C.byref(ctx.args),
             None if g_rho_c is None else g_rho_c.data_ptr(),

@@ -146,6 +146,7 @@ class LBMPipeNode(SimulationNode):
         self._storage = storage
         self._io_dtype = torch.float64 if storage == "f64" else torch.float32
         self._device = torch.device(device) if device is not None else None
+        self._dev_ready = False
         r, _, _ = _cross_section_radius(ny, nz)
         max_r = pipe_radius * min(ny, nz) / 2.0
         cross_wall = r >= np.float32(max_r)
@@ -182,10 +183,12 @@ class LBMPipeNode(SimulationNode):
         raise NotImplementedError("LBMPipeNode uses a discrete lattice Boltzmann update")
 
     def _dev(self) -> torch.device:
-        if not torch.cuda.is_available():
-            raise RuntimeError("LBMPipeNode needs a CUDA device (sm_100a); there is no CPU path")
-        if self._device is None:
-            self._device = torch.device("cuda", torch.cuda.current_device())
+        if not self._dev_ready:  # asked once: a CUDA device does not go away
+            if not torch.cuda.is_available():
+                raise RuntimeError("LBMPipeNode needs a CUDA device (sm_100a); there is no CPU path")
+            if self._device is None:
+                self._device = torch.device("cuda", torch.cuda.current_device())
+            self._dev_ready = True
         return self._device
 
     def _on(self, dev, key, arr):
@@ -258,7 +261,7 @@ class LBMPipeNode(SimulationNode):
         shape = (self._nx, self._ny, self._nz)
 
         def field(key, tail):
-            t = torch.as_tensor(state[key], device=dev).to(self._io_dtype).contiguous()
+            t = _lib.tensor_on(state[key], dev).to(self._io_dtype).contiguous()
             if tuple(t.shape) != shape + tail:
                 raise ValueError(f"state[{key!r}] shape {tuple(t.shape)} != {shape + tail}")
             return t
@@ -290,10 +293,9 @@ class LBMPipeNode(SimulationNode):
         m = _lib.lbm_moments()
         m.density, m.velocity = rho.data_ptr(), vel.data_ptr()
         lib = _lib_pipe()
-        nb = C.c_size_t()
-        _lib.check(lib.lbm_pipe_workspace_bytes(self._plan.handle, C.byref(nb)))
-        ws = torch.empty(int(nb.value), dtype=torch.uint8, device=dev)
-        stream = torch.cuda.current_stream(dev).cuda_stream
+        ws = torch.empty(self._plan._size(lib.lbm_pipe_workspace_bytes), dtype=torch.uint8,
+                         device=dev)
+        stream = _lib.raw_stream(dev)
         _lib.check(lib.lbm_pipe_rollout(self._plan.handle, stream, f.data_ptr(), f_out.data_ptr(),
                                         g.data_ptr(), g_out.data_ptr(), int(n_steps), C.byref(a),
                                         C.byref(m), tracer.data_ptr(), ws.data_ptr(), ws.numel()))
