@@ -38,7 +38,7 @@ int run_pipe(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_i
   int rc;
   bool done = false;
   if constexpr (std::is_same<S, float>::value) {
-    if (n == 1 && tiled_ok<S>(p, a, ws, true)) {
+    if (n == 1 && tiled_form<S>(p, a, ws, true) == kTiledBulk) {
       lbm::StepArgs m = a;
       m.mflags &= ~lbm::kMomRawVelocity;
       if (m.vel == nullptr) m.vel = ws + 2 * sb + 2 * tb;

@@ -44,6 +44,20 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
       : "memory");
 }
 
+// Four bytes of global memory -> this CTA's shared memory, completed through
+// word_copies_arrive.
+__device__ __forceinline__ void word_copy_g2s(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src)
+               : "memory");
+}
+
+// One arrival on `bar` (counted in its expected arrivals) once all earlier
+// word copies of this thread have landed.
+__device__ __forceinline__ void word_copies_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar))
+               : "memory");
+}
+
 // Two runs of this CTA's shared memory -> global (the second one may be empty),
 // sizes multiples of 16, addresses 16-byte aligned; tracked as one bulk
 // async-group of the issuing thread, which this call commits.

@@ -248,18 +248,20 @@ int run_steps(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_
   a.f_out = f_out;
   int rc;
   if constexpr (sizeof(typename lbm::StoreT<S>::IO) == 4) {
-    if (n == 1 && tiled_ok<S>(p, a, ws, true)) {
+    const TiledForm form = n == 1 ? tiled_form<S>(p, a, ws, true) : kTiledNone;
+    if (form != kTiledNone) {
       // the whole update in one pass; the workspace holds only the status word
       a.status = reinterpret_cast<int*>(ws);
       rc = cuda_check(cudaMemsetAsync(a.status, 0, sizeof(int), s), "cudaMemsetAsync");
       if (rc) return rc;
-      return launch_tiled<Q, S, lbm::kOutAoS>(p, a, s);
+      return form == kTiledBulk ? launch_tiled<Q, S, lbm::kOutAoS>(p, a, s)
+                                : launch_tiled_words<Q, S>(p, a, s);
     }
   }
   a.pout = A;
   lbm::StepArgs m = a;  // the first pass and intermediate steps write no moments
   m.rho = m.vel = m.prs = nullptr;
-  const bool tiled = n > 1 && tiled_ok<S>(p, a, ws + 2 * sb, false);
+  const bool tiled = n > 1 && tiled_form<S>(p, a, ws + 2 * sb, false) == kTiledBulk;
   if (tiled) {
     m.status = reinterpret_cast<int*>(ws + 2 * sb);
     rc = cuda_check(cudaMemsetAsync(m.status, 0, sizeof(int), s), "cudaMemsetAsync");

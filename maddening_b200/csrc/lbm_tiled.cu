@@ -43,9 +43,10 @@ lbm::TileGeo tile_geo(const lbm_plan* p, uint32_t grid) {
   return t;
 }
 
-template <int Q, class S, int MODE, bool FACES, bool FORCE, bool PIPE = false>
+template <int Q, class S, int MODE, bool FACES, bool FORCE, bool PIPE = false,
+          bool WORDS = false>
 int launch_tiled_t(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s) {
-  auto kern = lbm::k_tiled<Q, S, MODE, FACES, FORCE, PIPE>;
+  auto kern = lbm::k_tiled<Q, S, MODE, FACES, FORCE, PIPE, WORDS>;
   constexpr size_t smem = lbm::tiled_smem_bytes<Q, MODE>();
   int rc = cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            static_cast<int>(smem)),
@@ -88,6 +89,21 @@ int launch_tiled(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s) {
 }
 
 template <int Q, class S>
+int launch_tiled_words(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s) {
+  if constexpr (Q == 9) {
+    constexpr int M = lbm::kOutAoS;
+    const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
+    const bool force = a.force_mode != 0;
+    if (faces) return force ? launch_tiled_t<Q, S, M, true, true, false, true>(p, a, s)
+                            : launch_tiled_t<Q, S, M, true, false, false, true>(p, a, s);
+    return force ? launch_tiled_t<Q, S, M, false, true, false, true>(p, a, s)
+                 : launch_tiled_t<Q, S, M, false, false, false, true>(p, a, s);
+  } else {
+    return fail(LBM_ERR_UNSUPPORTED, "the word-copy one-pass update is D2Q9");
+  }
+}
+
+template <int Q, class S>
 int launch_tiled_pipe(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s) {
   if constexpr (Q == 19 && std::is_same<S, float>::value)
     return launch_tiled_t<Q, S, lbm::kOutAoS, false, false, true>(p, a, s);
@@ -100,5 +116,6 @@ int launch_tiled_pipe(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s)
                                                 cudaStream_t);                           \
   template int launch_tiled<Q, S, lbm::kOutState>(const lbm_plan*, const lbm::StepArgs&, \
                                                   cudaStream_t);                          \
+  template int launch_tiled_words<Q, S>(const lbm_plan*, const lbm::StepArgs&, cudaStream_t); \
   template int launch_tiled_pipe<Q, S>(const lbm_plan*, const lbm::StepArgs&, cudaStream_t);
 LBM_TILED_INST(LBM_UNIT_Q, LBM_UNIT_S)

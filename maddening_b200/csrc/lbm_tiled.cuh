@@ -35,9 +35,10 @@
 // D3Q19 FP32; the halo re-reads hit L2.  The arithmetic is the two-pass
 // path's operation for operation, so the outputs are bit-identical to it.
 //
-// Requirements (checked on the host): 32-bit IO (FP32, FP16 or BF16
-// storage), an a2 extent that is a multiple of 4, f_in (and f_out for
-// kOutAoS) 16-byte aligned and not overlapping, no halo-padded block.  Every wait is bounded in time and also ends when another warp
+// Requirements (checked on the host): 32-bit IO (FP32, FP16 or BF16 storage),
+// f_in and f_out not overlapping, no halo-padded block; the bulk copies want an
+// a2 extent that is a multiple of 4 and f_in (and f_out for kOutAoS) 16-byte
+// aligned, the word-copy form (D2Q9 update) neither.  Every wait is bounded in time and also ends when another warp
 // has given up; then the block sets bit 0 of *status, waits (bounded) for its
 // own copies in flight and returns.
 #pragma once
@@ -232,6 +233,34 @@ __device__ __forceinline__ void collide_ref(const StepArgs& a, uint32_t c, float
   }
 }
 
+// The same without any alignment (rows that are not groups of four cells, an
+// f_in off 16-byte boundaries), for one-row tiles: the warp copies the buffered
+// row word by word, the wrapped halo cells as pieces of their own, into the same
+// places.
+template <int Q>
+__device__ __forceinline__ void tiled_issue_words(const StepArgs& a, const TileGeo& t,
+                                                  const PlaneRef& p, float* buf, uint64_t* bar,
+                                                  uint32_t lane) {
+  using T = TileShape<Q>;
+  static_assert(T::RP == 1, "one buffered row per plane");
+  if (t.no_copy) return;
+  const uint32_t n2 = a.g.n2;
+  const bool wrap_l = p.z0 == 0, wrap_r = p.z0 + p.tzv == n2;
+  const uint32_t b = p.z0 * Q - (wrap_l ? 0u : Q);
+  const uint32_t e = (p.z0 + p.tzv) * Q + (wrap_r ? 0u : Q);
+  const float* row = static_cast<const float*>(a.f_in) +
+                     static_cast<size_t>(plane_s(t, p)) * t.SS * Q;
+  float* dst = buf + (T::LCH - Q);  // the cell before the tile
+  if (wrap_l && lane < Q) word_copy_g2s(dst + lane, row + (n2 - 1) * Q + lane);
+  if (wrap_r && lane < Q) word_copy_g2s(dst + (1 + p.tzv) * Q + lane, row + lane);
+  const float* const src = row + b + lane;
+  float* const dl = dst + (wrap_l ? Q : 0) + lane;
+#pragma unroll 8
+  for (uint32_t i = 0; i < (T::CW * Q + 31) / 32; ++i)
+    if (lane + i * 32 < e - b) word_copy_g2s(dl + i * 32, src + i * 32);
+  word_copies_arrive(bar);
+}
+
 // collide_ref for the two cells of a lane (c0, c1), two-wide arithmetic.
 template <int Q, class S, bool FORCE>
 __device__ __forceinline__ void collide_ref2(const StepArgs& a, uint32_t c0, uint32_t c1,
@@ -420,7 +449,9 @@ struct Ring {
 };
 
 // PIPE: the pipe node's force (force mode 3), f_bc and moments out, no faces.
-template <int Q, class S, int MODE, bool FACES, bool FORCE, bool PIPE = false>
+// WORDS: no alignment of rows and buffers -- planes come in word by word
+// (tiled_issue_words) and f_bc leaves the staging rows by plain stores.
+template <int Q, class S, int MODE, bool FACES, bool FORCE, bool PIPE = false, bool WORDS = false>
 __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
     k_tiled(const __grid_constant__ StepArgs a, const __grid_constant__ TileGeo t) {
   using T = TileShape<Q>;
@@ -442,7 +473,7 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
 
   if (tid == 0) {
     for (uint32_t s = 0; s < S_; ++s) {
-      mbar_init(&sync->full[s], 1);
+      mbar_init(&sync->full[s], WORDS ? 32 : 1);
       mbar_init(&sync->collided[s], T::NCW);
       mbar_init(&sync->consumed[s], T::NOW);
     }
@@ -463,8 +494,9 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
           P < S_ || tile_wait(&sync->consumed[r.s], r.par ^ 1u, t.wait_ns, abort);
       if (!__all_sync(0xffffffffu, ok)) break;
       fence_proxy_async_smem();
-      tiled_issue<Q>(a, t, L, planes + static_cast<size_t>(r.s) * T::PLANE, &sync->full[r.s],
-                     lane);
+      float* buf = planes + static_cast<size_t>(r.s) * T::PLANE;
+      if constexpr (WORDS) tiled_issue_words<Q>(a, t, L, buf, &sync->full[r.s], lane);
+      else tiled_issue<Q>(a, t, L, buf, &sync->full[r.s], lane);
     }
     if (lane == 0) sync->issued = P;
   } else if (warp <= static_cast<uint32_t>(T::NCW)) {
@@ -668,7 +700,7 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
       const Mom<V> mo = moments<Q, V, FORCE>(d, F, true);
       if constexpr (MODE == kOutAoS) {
         // this warp's earlier store has read the staging rows
-        if (lane == 0) bulk_wait_read();
+        if (!WORDS && lane == 0) bulk_wait_read();
         __syncwarp();
         float* row = wst + lane * Q;
 #pragma unroll
@@ -682,9 +714,23 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
         // moments, so that it waits only for the staging writes.
         const uint32_t n0 = __popc(__ballot_sync(0xffffffffu, act0));
         const uint32_t n1 = kTwo ? __popc(__ballot_sync(0xffffffffu, act1)) : 0u;
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0 && n0 > 0) {
+        if constexpr (WORDS) {
+          __syncwarp();
+          // (lane 0 has the run's first cell where there is one)
+          float* out = static_cast<float*>(a.f_out) +
+                       static_cast<size_t>(__shfl_sync(0xffffffffu, x.c, 0)) * Q;
+#pragma unroll
+          for (uint32_t i = 0; i < Q; ++i) {
+            const uint32_t w = i * 32 + lane;
+            if (w < n0 * Q) out[w] = wst[w];
+            if (kTwo && w < n1 * Q) out[T::OZ * Q + w] = wst[32 * Q + w];
+          }
+          __syncwarp();
+        } else {
+          fence_proxy_async_smem();
+          __syncwarp();
+        }
+        if (!WORDS && lane == 0 && n0 > 0) {
           float* out = static_cast<float*>(a.f_out) + static_cast<size_t>(x.c) * Q;
           bulk_store2_s2g(out, wst, n0 * Q * 4, out + T::OZ * Q, wst + 32 * Q, n1 * Q * 4);
         }
@@ -735,7 +781,7 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
         }
       }
     }
-    if constexpr (MODE == kOutAoS) {
+    if constexpr (MODE == kOutAoS && !WORDS) {
       if (lane == 0) bulk_wait_all();
     }
   }

@@ -26,7 +26,7 @@ Additions beyond the reference (documented extensions):
   form gives bit-identical results.
 * ``one_pass`` -- ``update`` (and the first step of ``run``) reads the
   reference-layout ``f`` once in a tiled kernel (``None`` or ``True``, the
-  default; FP32, FP16 and BF16 storage, last extent a multiple of 4) or runs
+  default; FP32, FP16 and BF16 storage; D3Q19: last extent a multiple of 4) or runs
   as two passes (``False``); the results are bit-identical.
 """
 
