@@ -23,18 +23,26 @@ void launch_step_mode(const lbm::StepArgs& a, cudaStream_t s) {
   }
 }
 
-// Paired-cell state step (lbm_pair.cuh): the default for 16-bit storage,
-// opt-in for FP32 (LBM_PLAN_PAIRED_CELLS), off with LBM_PLAN_SINGLE_CELLS.
-// Rows of even length (row segments when they split into warps of 64 cells,
-// instance-wide pairs otherwise); state planes and the wall mask aligned for
+// Paired-cell state step (lbm_pair.cuh): the default for 16-bit storage; for FP32
+// without faces, or on lattices large enough that the faces' own code is few
+// warps' work; always with LBM_PLAN_PAIRED_CELLS, never with
+// LBM_PLAN_SINGLE_CELLS.  FP32 us a step with two cells / one cell per thread,
+// force without faces: 48^3 2.97 / 4.27, 96^3 19.9 / 22.7, 256^3 379 / 392, 1024^2
+// 8.4 / 12.4, 2048^2 48.4 / 50.9; with faces: 64^3 8.1 / 7.6, 96^3 23.3 / 23.9,
+// 128^3 53.6 / 53.1, 160^3 100.1 / 100.8, 256^3 383 / 393; 512^2 4.6 / 4.5, 1024^2
+// 9.9 / 12.6.  Rows of even length; state planes and the wall mask aligned for
 // the pair width.
-template <class S>
+template <int Q, class S>
 bool pair_ok(const lbm_plan* p, const lbm::StepArgs& a) {
   if constexpr (sizeof(S) == 8) {
     return false;
   } else {
     if (p->flags & LBM_PLAN_SINGLE_CELLS) return false;
-    if (sizeof(S) == 4 && !(p->flags & LBM_PLAN_PAIRED_CELLS)) return false;
+    if (sizeof(S) == 4 && !(p->flags & LBM_PLAN_PAIRED_CELLS)) {
+      const bool faces =
+          a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
+      if (faces && p->g.ncell < (Q == 9 ? 1u << 20 : 1u << 22)) return false;
+    }
     const uintptr_t al = 2 * sizeof(S);
     return p->g.n2 % 2 == 0 && reinterpret_cast<uintptr_t>(a.pin) % al == 0 &&
            reinterpret_cast<uintptr_t>(a.pout) % al == 0 &&
@@ -149,9 +157,10 @@ int launch_pair(const lbm::StepArgs& a, cudaStream_t s) {
         return cuda_check(cudaGetLastError(), "k_step_gquad launch");
       }
     }
+    // row segments in blocks of two or four warps, else instance-wide pairs (192^3
+    // FP16 107 us a step against 122 in one-warp blocks, 320^3 482 / 552)
     if (a.g.n2 % 256 == 0) launch_pair_w<Q, S, 4>(a, s);
     else if (a.g.n2 % 128 == 0) launch_pair_w<Q, S, 2>(a, s);
-    else if (a.g.n2 % 64 == 0) launch_pair_w<Q, S, 1>(a, s);
     else launch_gpair<Q, S, false>(a, s);
     return cuda_check(cudaGetLastError(), "k_step_pair launch");
   }
@@ -206,7 +215,7 @@ int launch_state_step(const lbm_plan* p, const lbm::StepArgs& m, cudaStream_t s)
       return cuda_check(cudaGetLastError(), "k_step_gpair launch");
     }
   }
-  if (pair_ok<S>(p, m)) return launch_pair<Q, S>(m, s);
+  if (pair_ok<Q, S>(p, m)) return launch_pair<Q, S>(m, s);
   return launch_step<Q, S>(m, false, s);
 }
 
