@@ -759,9 +759,10 @@ int lbm_batch_create(const lbm_plan* const* plans, int32_t n, lbm_batch** out) {
       return fail(LBM_ERR_INVALID, "instance %d: padded rows exceed 32-bit indexing", i);
     }
     b->sgeo.push_back(g);
-    for (uint32_t c = 0; c < g.ncell; c += lbm::kBatchTile)
+    const uint32_t tile = lbm::batch_tile(p->elem);
+    for (uint32_t c = 0; c < g.ncell; c += tile)
       per[i].push_back(lbm::BatchTile{static_cast<uint32_t>(i), c});
-    for (uint32_t c = 0; c < g.pstride; c += lbm::kBatchTile)
+    for (uint32_t c = 0; c < g.pstride; c += tile)
       sper[i].push_back(lbm::BatchTile{static_cast<uint32_t>(i), c});
     ntiles += per[i].size();
     nstiles += sper[i].size();

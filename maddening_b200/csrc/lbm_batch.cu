@@ -16,12 +16,12 @@ void batched_launch(bool pair, bool pad, const lbm::StepArgs* args, const lbm::B
                     uint32_t nt, unsigned grid, int which, cudaStream_t s) {
   if constexpr (MODE == lbm::kOutState && sizeof(S) == 2) {
     if (pair) {
-      if (pad) launch_after(lbm::k_batched_pair<Q, S, SPEC, true>, grid, lbm::kBlock, s, args, t, nt, which);
-      else launch_after(lbm::k_batched_pair<Q, S, SPEC, false>, grid, lbm::kBlock, s, args, t, nt, which);
+      if (pad) lbm::k_batched_pair<Q, S, SPEC, true><<<grid, lbm::kBlock, 0, s>>>(args, t, nt, which);
+      else lbm::k_batched_pair<Q, S, SPEC, false><<<grid, lbm::kBlock, 0, s>>>(args, t, nt, which);
       return;
     }
   }
-  launch_after(lbm::k_batched_step<Q, S, MODE, SPEC>, grid, lbm::kBlock, s, args, t, nt, which);
+  lbm::k_batched_step<Q, S, MODE, SPEC><<<grid, lbm::kBlock, 0, s>>>(args, t, nt, which);
 }
 
 // spec: 0 = per-tile run-time choice, else 1 + 2 FACES + FORCE shared by all members

@@ -1009,16 +1009,12 @@ __global__ void __launch_bounds__(kBlock, min_blocks<S>())
 // Batched ensemble: many lattices (own shape, tau, force, walls) in one launch
 // ---------------------------------------------------------------------------
 
-// A tile is kBatchTile consecutive cells of one instance (a multiple of
-// 2 kBlock: the paired kernel gives each thread kBatchTile / (2 kBlock) pairs).
-// 512 cells: on the 64-lattice ensemble 37.4k (FP32) and 54.8k (FP16) MLUPS
-// against 36.7k / 52.6k for 256-cell tiles, 36.6k / 55.0k for 1024 and
-// 36.0k / 53.1k for 2048 (B200).
-#ifndef LBM_BATCH_TILE
-#define LBM_BATCH_TILE (4 * LBM_STEP_BLOCK)
-#endif
-constexpr int kBatchTile = LBM_BATCH_TILE;
-static_assert(kBatchTile % (2 * kBlock) == 0, "batch tiles hold whole pair rows of a block");
+// A tile is batch_tile(bytes per population) consecutive cells of one instance (a
+// multiple of 2 kBlock: the paired kernel gives each thread whole pairs of it).
+// On the 64-lattice ensemble (B200): FP32, one cell per thread, 37.4k MLUPS with
+// 512 cells against 36.7k / 36.6k / 36.0k with 256 / 1024 / 2048; FP16, two cells
+// per thread, 590 us a step with 1024 cells against 593 / 596 with 768 / 512.
+constexpr int batch_tile(size_t elem) { return (elem == 2 ? 8 : 4) * kBlock; }
 struct BatchTile {
   uint32_t inst;
   uint32_t first;
@@ -1060,13 +1056,11 @@ template <int Q, class S, int MODE, int SPEC>
 __global__ void __launch_bounds__(kBlock, batched_min_blocks<S>())
     k_batched_step(const StepArgs* __restrict__ args, const BatchTile* __restrict__ tiles,
                    uint32_t ntiles, int which) {
-  grid_launch_next();
-  grid_wait_previous();
   for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const BatchTile tile = tiles[t];
     const StepArgs& sa = args[kBatchArgs * tile.inst + which];
 #pragma unroll 1
-    for (int j = 0; j < kBatchTile / kBlock; ++j) {
+    for (int j = 0; j < batch_tile(sizeof(S)) / kBlock; ++j) {
       const uint32_t first = tile.first + j * kBlock;  // block-uniform
       if (first >= sa.g.ncell) break;
       const uint32_t c = first + threadIdx.x;
@@ -1096,7 +1090,7 @@ __global__ void __launch_bounds__(kBlock, batched_min_blocks<S>())
       cur = tile.inst;
     }
 #pragma unroll 1
-    for (int j = 0; j < kBatchTile / kBlock; ++j) {
+    for (int j = 0; j < batch_tile(sizeof(S)) / kBlock; ++j) {
       const uint32_t first = tile.first + j * kBlock;  // block-uniform
       if (first >= sa.g.ncell) break;
       const uint32_t c = first + threadIdx.x;

@@ -481,20 +481,23 @@ __global__ void __launch_bounds__(kBlock, kPairMinWarps / (kBlock / 32))
   gpair_step<Q, S, FACES, FORCE, PAD>(a, blockIdx.x * kBlock + threadIdx.x);
 }
 
+// Register budget of the batched pairs (64 lattices FP16): 24 warps 596 us a step
+// (512-cell tiles), 28: 600, 20: 621; the member's arguments in shared memory 620,
+// programmatic launches 604.
+constexpr int kBatchPairWarps = 24;
+
 // Batched ensemble, state steps of members with even rows: a tile of
-// kBatchTile cells is kBatchTile / 2 pairs, kBatchTile / (2 kBlock) per thread
+// batch_tile cells is half as many pairs, batch_tile / (2 kBlock) per thread
 // (see k_batched_step for the tile walk and SPEC).
 template <int Q, class S, int SPEC, bool PAD>
-__global__ void __launch_bounds__(kBlock, kPairMinWarps / (kBlock / 32))
+__global__ void __launch_bounds__(kBlock, kBatchPairWarps / (kBlock / 32))
     k_batched_pair(const StepArgs* __restrict__ args, const BatchTile* __restrict__ tiles,
                    uint32_t ntiles, int which) {
-  grid_launch_next();
-  grid_wait_previous();
   for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const BatchTile tile = tiles[t];
     const StepArgs& sa = args[kBatchArgs * tile.inst + which];
 #pragma unroll 1
-    for (int j = 0; j < kBatchTile / (2 * kBlock); ++j) {
+    for (int j = 0; j < batch_tile(sizeof(S)) / (2 * kBlock); ++j) {
       const uint32_t pidx = (tile.first >> 1) + j * kBlock + threadIdx.x;
       // whole warps past the member's last pair skip the step; a partial warp
       // runs it with its extra lanes clamped
