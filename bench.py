@@ -55,18 +55,18 @@ GRID = (256, 256, 256)
 TAU = 0.6
 U_IN = (0.05, 0.0, 0.0)
 BYTES_PER_CELL = 152  # D3Q19 FP32: 19 x 4 B read + 19 x 4 B written
-# DRAM bytes of one state step launch (k_step<19, float>) of the 256^3 FP32
+# DRAM bytes of one state step launch (k_step_pair<19, float>) of the 256^3 FP32
 # workload, from one capture of
 #   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum
-#       --clock-control none -k regex:k_step -s 5 -c 3 python bench.py --steps 20 --warmup 3
+#       --clock-control none -k regex:k_step_pair -s 5 -c 2 python bench.py --steps 20 --warmup 3
 #       --no-cpu-baseline --no-variants
 # (one pass): 1.29 GB read + 1.22 GB written per launch, against 2.55 GB
 # algorithmic (the remainder of the writes is still in L2 when the launch ends).
-NCU_TRAFFIC_256_F32 = 2.51e9
+NCU_TRAFFIC_256_F32 = 2.516e9
 METRIC = "MLUPS (D3Q19 FP32 lattice updates/s) & HBM roofline fraction"
 # the state-step kernel each storage form runs on the workload (rows of 256 cells)
 KERNEL_LABEL = {
-    "f32": "k_step<19,float,kOutState,faces,no force> (fused pull-stream-collide, one cell "
+    "f32": "k_step_pair<19,float,faces,no force,4> (fused pull-stream-collide, two cells "
            "per thread)",
     "f64": "k_step<19,double,kOutState,faces,no force> (one cell per thread)",
     "f16": "k_step_quad<19,__half,faces,no force,2> (four cells per thread, 64-bit words)",

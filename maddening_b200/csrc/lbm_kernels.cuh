@@ -19,11 +19,10 @@
 // outputs) and collides again, writing p for the next step: 19 loads and 19
 // stores per cell, each warp access one contiguous 32-element run.
 //
-// One thread owns one cell.  For FP32 storage this beat 2- and 4-cell vector
-// forms on B200: the wider forms need more registers than 32 resident warps
-// per SM allow, and the lost occupancy costs more than the wider accesses save.
-// 16-bit storage moves too few bytes per cell for that: it takes two or four
-// cells per thread (lbm_pair.cuh) and rounds stochastically (below).
+// One thread owns one cell here.  Two or four cells per thread (lbm_pair.cuh), with
+// two-wide FP32 arithmetic, take the 16-bit storages, which also round
+// stochastically (below), and FP32 where they are faster; FP64, the outputs in
+// the reference layout and the recorded steps stay with this form.
 #pragma once
 
 #include <cuda_bf16.h>

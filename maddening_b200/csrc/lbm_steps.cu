@@ -9,17 +9,22 @@
 
 namespace {
 
-template <int Q, class S, int MODE>
+// AFTER: as a step of a rollout on one stream (launch_after).
+template <int Q, class S, int MODE, bool AFTER = true>
 void launch_step_mode(const lbm::StepArgs& a, cudaStream_t s) {
   const unsigned grid = grid_for(a.cell_end - a.cell0);
   const bool faces = a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
   const bool force = a.force_mode != 0;
+  auto launch = [&](void (*kern)(const lbm::StepArgs)) {
+    if constexpr (AFTER) launch_after(kern, grid, lbm::kBlock, s, a);
+    else kern<<<grid, lbm::kBlock, 0, s>>>(a);
+  };
   if (faces) {
-    if (force) launch_after(lbm::k_step<Q, S, MODE, true, true>, grid, lbm::kBlock, s, a);
-    else launch_after(lbm::k_step<Q, S, MODE, true, false>, grid, lbm::kBlock, s, a);
+    if (force) launch(lbm::k_step<Q, S, MODE, true, true>);
+    else launch(lbm::k_step<Q, S, MODE, true, false>);
   } else {
-    if (force) launch_after(lbm::k_step<Q, S, MODE, false, true>, grid, lbm::kBlock, s, a);
-    else launch_after(lbm::k_step<Q, S, MODE, false, false>, grid, lbm::kBlock, s, a);
+    if (force) launch(lbm::k_step<Q, S, MODE, false, true>);
+    else launch(lbm::k_step<Q, S, MODE, false, false>);
   }
 }
 
@@ -369,7 +374,9 @@ template <int Q, class S>
 int state_op(StateOp op, const lbm::StepArgs& a, cudaStream_t s) {
   if (op == kFromF) return launch_prepare<Q, S>(a, s);
   if (op == kStep) {
-    launch_step_mode<Q, S, lbm::kOutState>(a, s);  // one cell per thread, any storage
+    // one cell per thread, any storage; an ordinary launch: the caller orders these
+    // steps against exchanges on other streams
+    launch_step_mode<Q, S, lbm::kOutState, false>(a, s);
     return cuda_check(cudaGetLastError(), "k_step launch");
   }
   return launch_step<Q, S>(a, true, s);
