@@ -143,7 +143,10 @@ def tensor_on(x, dev):
 
 
 def raw_stream(dev) -> int:
-    """Handle of the current stream of ``dev``."""
+    """Handle of the current stream of ``dev``; a device that is not a CUDA device
+    is refused (its tensors must not reach a launch)."""
+    if dev.type != "cuda":
+        raise ValueError(f"Expected a cuda device, but got: {dev}")
     index = dev.index
     return torch._C._cuda_getCurrentRawStream(
         torch.cuda.current_device() if index is None else index)
