@@ -135,10 +135,35 @@ __host__ __device__ constexpr size_t tiled_stage_bytes() {
              ? static_cast<size_t>(TileShape<Q>::NOW) * 32 * TileShape<Q>::CPO * Q * 4
              : 0;
 }
+// Shared memory: the ring, the staging rows, kIdleWords words, TileSync.
+constexpr uint32_t kIdleWords = 32;
+template <int Q, int MODE>
+__host__ __device__ constexpr uint32_t tiled_idle_word() {
+  return Sweep<Q>::SLOTS * TileShape<Q>::PLANE +
+         static_cast<uint32_t>(tiled_stage_bytes<Q, MODE>() / 4);
+}
 template <int Q, int MODE>
 __host__ __device__ constexpr size_t tiled_smem_bytes() {
-  return static_cast<size_t>(Sweep<Q>::SLOTS) * TileShape<Q>::PLANE * 4 +
-         tiled_stage_bytes<Q, MODE>() + sizeof(TileSync<Q>);
+  return static_cast<size_t>(tiled_idle_word<Q, MODE>() + kIdleWords) * 4 + sizeof(TileSync<Q>);
+}
+
+// Place of collide cell m (row m / CW, cell m % CW of a plane's buffered cells) in
+// a tile of tyv x tzv cells: its word in slot 0 and the words from a slot to the
+// next.  Without such a cell in the tile the lane reads the idle words instead,
+// the same in every slot, which nothing writes once the block has started: the
+// value is thrown away, but any cell of the plane is one that another warp may be
+// overwriting.
+struct CollidePlace {
+  uint32_t word, step;
+};
+template <int Q, int MODE>
+__host__ __device__ constexpr CollidePlace collide_place(uint32_t m, uint32_t tyv, uint32_t tzv) {
+  using T = TileShape<Q>;
+  static_assert(Q <= static_cast<int>(kIdleWords), "the idle words hold one cell");
+  const uint32_t rr = m / T::CW, cc = m % T::CW;
+  if (rr < tyv + 2 * T::HR && cc < tzv + 2)
+    return {rr * T::RW + (T::LCH - Q) + cc * Q, static_cast<uint32_t>(T::PLANE)};
+  return {tiled_idle_word<Q, MODE>(), 0u};
 }
 
 // Host-computed geometry of the sweep.
@@ -465,7 +490,7 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
   float* planes = reinterpret_cast<float*>(smem);
   float* stage = planes + static_cast<size_t>(S_) * T::PLANE;
   TileSync<Q>* sync = reinterpret_cast<TileSync<Q>*>(
-      smem + static_cast<size_t>(S_) * T::PLANE * 4 + tiled_stage_bytes<Q, MODE>());
+      smem + static_cast<size_t>(tiled_idle_word<Q, MODE>() + kIdleWords) * 4);
   volatile int* abort = &sync->abort;
   const Geo& g = a.g;
   const uint32_t tid = threadIdx.x;
@@ -481,6 +506,7 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
     sync->issued = 0;
     fence_mbar_init();
   }
+  if (tid < kIdleWords) planes[tiled_idle_word<Q, MODE>() + tid] = 0.0f;
   __syncthreads();
 
   if (warp == 0) {
@@ -503,16 +529,8 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
     // ---- collide warps: plane P in place once it has landed, two cells per
     // lane; the wall bits of its cells go to the plane's words
     const uint32_t j = warp - 1;
-    uint32_t rr[2], cc[2], soff[2], rz[2];
-    bool mine[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const uint32_t m = (2 * j + k) * 32 + lane;
-      rr[k] = m / T::CW;
-      cc[k] = m % T::CW;
-      mine[k] = false;
-      soff[k] = rz[k] = 0;
-    }
+    uint32_t rz[2] = {0, 0};
+    CollidePlace at[2] = {};
     PlaneRef C;
     plane_first<Q>(a, t, blockIdx.x, C);
     Ring<Q> r;
@@ -522,10 +540,11 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
         item = C.item;
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          mine[k] = rr[k] < C.tyv + 2 * T::HR && cc[k] < C.tzv + 2;
-          // a lane without a cell runs the plane's first one and stores nothing
-          const uint32_t ry = mine[k] ? rr[k] : 0u, cz = mine[k] ? cc[k] : 0u;
-          soff[k] = ry * T::RW + (T::LCH - Q) + cz * Q;
+          const uint32_t m = (2 * j + k) * 32 + lane;
+          at[k] = collide_place<Q, MODE>(m, C.tyv, C.tzv);
+          // a lane without a cell takes the index of the plane's first one
+          const bool mine = at[k].step != 0;
+          const uint32_t ry = mine ? m / T::CW : 0u, cz = mine ? m % T::CW : 0u;
           rz[k] = wrapu(static_cast<int>(C.y0 + ry) - T::HR, t.NR) * t.SR +
                   wrapu(static_cast<int>(C.z0 + cz) - 1, g.n2);
         }
@@ -538,12 +557,13 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
       }
       const bool ok = tile_wait(&sync->full[r.s], r.par, t.wait_ns, abort);
       if (!__all_sync(0xffffffffu, ok)) break;
-      float* slot = planes + static_cast<size_t>(r.s) * T::PLANE;
+      float* const c0 = planes + (at[0].word + r.s * at[0].step);
+      float* const c1 = planes + (at[1].word + r.s * at[1].step);
       // No branch around this body: given one per cell, the compiler splits it
       // by which cells a lane owns and a warp runs it up to three times.
       F2 d[Q];
 #pragma unroll
-      for (int q = 0; q < Q; ++q) d[q] = F2(slot[soff[0] + q], slot[soff[1] + q]);
+      for (int q = 0; q < Q; ++q) d[q] = F2(c0[q], c1[q]);
 #pragma unroll
       for (int q = 0; q < Q; ++q) d[q] = to_offset<Q, F2>(d[q], q);
       if constexpr (PIPE)
@@ -553,8 +573,8 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
       __syncwarp();
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
-        if (mine[0]) slot[soff[0] + q] = d[q].v.x;
-        if (mine[1]) slot[soff[1] + q] = d[q].v.y;
+        if (at[0].step != 0) c0[q] = d[q].v.x;
+        if (at[1].step != 0) c1[q] = d[q].v.y;
       }
       const uint32_t w0 = __ballot_sync(0xffffffffu, wb[0] != 0);
       const uint32_t w1 = __ballot_sync(0xffffffffu, wb[1] != 0);
