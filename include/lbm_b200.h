@@ -101,7 +101,7 @@ typedef struct {
                                 its barriers but issues no copies and gives up a
                                 wait after 0.2 ms (instead of 2 s), so its waits
                                 run out: it sets the status word and returns
-                                early with the outputs incomplete.  Only for
+                                early with NaN in its outputs.  Only for
                                 testing the timeout path */
 
 typedef struct {
@@ -160,7 +160,13 @@ int lbm_equilibrium(const lbm_plan* plan, lbm_stream_t stream, const void* rho,
 
 /* One reference step, LBMNode.update (lbm.py:899-986): macroscopic with F/2,
  * BGK + Guo collide on every cell, periodic stream on every axis, wall-node
- * swap, inlet then outlet face, output moments (u = 0 in walls). */
+ * swap, inlet then outlet face, output moments (u = 0 in walls).
+ * The one-pass kernel behind this call, a single pipe step and the first step
+ * of a rollout bounds every wait in time (2 s).  A block whose wait runs out
+ * leaves NaN in all its output cells, so a broken result shows in the outputs
+ * (and in what later steps make of them), and sets a word that starts at 0:
+ * the first 4 bytes of the workspace of an update or a single pipe step, the
+ * word after the two state copies in a rollout's. */
 int lbm_update(const lbm_plan* plan, lbm_stream_t stream, const void* f_in,
                void* f_out, const lbm_step_args* args, const lbm_moments* out,
                void* workspace, size_t workspace_bytes);

@@ -40,7 +40,7 @@
 // a2 extent that is a multiple of 4 and f_in (and f_out for kOutAoS) 16-byte
 // aligned, the word-copy form (D2Q9 update) neither.  Every wait is bounded in time and also ends when another warp
 // has given up; then the block sets bit 0 of *status, waits (bounded) for its
-// own copies in flight and returns.
+// own copies in flight, fills its output cells with NaN and returns.
 #pragma once
 
 #include <type_traits>
@@ -473,6 +473,36 @@ struct Ring {
   }
 };
 
+// NaN in every output cell of this block's work items: what a block writes whose
+// waits ran out, so that an incomplete result shows in the results themselves
+// and in what later steps make of them, with no status to ask for.
+template <int Q, class S, int MODE>
+__device__ __noinline__ void tiled_mark_failed(const StepArgs& a, const TileGeo& t) {
+  constexpr int D = Lat<Q>::D;
+  const float nan = __uint_as_float(0x7fffffffu);
+  PlaneRef p;
+  for (uint32_t item = blockIdx.x; item < t.items; item += gridDim.x) {
+    plane_first<Q>(a, t, item, p);
+    for (uint32_t i = threadIdx.x; i < p.nv * p.tyv * p.tzv; i += blockDim.x) {
+      const uint32_t r = i / p.tzv;
+      const uint32_t c = (p.k0 + r / p.tyv) * t.SS + (p.y0 + r % p.tyv) * t.SR + p.z0 + i % p.tzv;
+      for (int q = 0; q < Q; ++q) {
+        if constexpr (MODE == kOutAoS) {
+          static_cast<float*>(a.f_out)[static_cast<size_t>(c) * Q + q] = nan;
+        } else if constexpr (sizeof(S) == 2) {  // NaN in both 16-bit formats
+          static_cast<unsigned short*>(a.pout)[static_cast<uint32_t>(q) * a.g.pstride + c] = 0x7fffu;
+        } else {
+          static_cast<float*>(a.pout)[static_cast<uint32_t>(q) * a.g.pstride + c] = nan;
+        }
+      }
+      if (a.rho != nullptr) static_cast<float*>(a.rho)[c] = nan;
+      if (a.prs != nullptr) static_cast<float*>(a.prs)[c] = nan;
+      if (a.vel != nullptr)
+        for (int d = 0; d < D; ++d) static_cast<float*>(a.vel)[static_cast<size_t>(c) * D + d] = nan;
+    }
+  }
+}
+
 // PIPE: the pipe node's force (force mode 3), f_bc and moments out, no faces.
 // WORDS: no alignment of rows and buffers -- planes come in word by word
 // (tiled_issue_words) and f_bc leaves the staging rows by plain stores.
@@ -806,14 +836,17 @@ __global__ void __launch_bounds__(TileShape<Q>::NT, Sweep<Q>::MINB)
     }
   }
 
-  __syncthreads();
-  if (tid == 0 && sync->abort) {
-    atomicOr(a.status, 1);
-    // the last copies issued may be in flight: wait for them (bounded) before exit
-    sync->abort = 0;
-    const uint32_t n = sync->issued;
-    for (uint32_t P = n > S_ ? n - S_ : 0; P < n; ++P)
-      if (!tile_wait(&sync->full[P % S_], (P / S_) & 1u, t.wait_ns, abort)) break;
+  // (the warp that gave up sees its own flag, so every thread learns of it here)
+  if (__syncthreads_or(*abort)) {
+    if (tid == 0) {
+      atomicOr(a.status, 1);
+      // the last copies issued may be in flight: wait for them (bounded) before exit
+      sync->abort = 0;
+      const uint32_t n = sync->issued;
+      for (uint32_t P = n > S_ ? n - S_ : 0; P < n; ++P)
+        if (!tile_wait(&sync->full[P % S_], (P / S_) & 1u, t.wait_ns, abort)) break;
+    }
+    tiled_mark_failed<Q, S, MODE>(a, t);
   }
 }
 
