@@ -104,6 +104,12 @@ typedef struct {
                                 early with NaN in its outputs.  Only for
                                 testing the timeout path */
 
+#define LBM_PLAN_ONE_PASS 128u /* the one-pass tiled kernel wherever it can run, also
+                                on the D2Q9 lattices (small ones, rows that fill
+                                few of its 252-cell tiles) on which two passes are
+                                faster; same results bit for bit.  Not together
+                                with LBM_PLAN_TWO_PASS */
+
 typedef struct {
   int32_t lattice;  /* lbm_lattice: 19 (D3Q19) or 9 (D2Q9)                */
   int32_t storage;  /* lbm_storage                                        */

@@ -41,6 +41,7 @@ PLAN_SINGLE_CELLS = 2
 PLAN_PAIRED_CELLS = 4
 PLAN_TWO_PASS = 8
 PLAN_TEST_WAIT_TIMEOUT = 16
+PLAN_ONE_PASS = 128
 
 
 class lbm_desc(C.Structure):

@@ -301,10 +301,13 @@ int lbm_plan_create(const lbm_desc* desc, lbm_plan** plan) {
   if (!(desc->tau > 0.5) || !std::isfinite(desc->tau))
     return fail(LBM_ERR_INVALID, "tau must be > 0.5 (got %g). Increase viscosity.", desc->tau);
   constexpr uint32_t kKnownFlags = LBM_PLAN_SINGLE_CELLS | LBM_PLAN_PAIRED_CELLS |
-                                   LBM_PLAN_TWO_PASS | LBM_PLAN_TEST_WAIT_TIMEOUT;
+                                   LBM_PLAN_TWO_PASS | LBM_PLAN_TEST_WAIT_TIMEOUT |
+                                   LBM_PLAN_ONE_PASS;
   if (desc->flags & ~kKnownFlags)
     return fail(LBM_ERR_INVALID, "unknown or reserved plan flags 0x%x",
                 static_cast<unsigned>(desc->flags & ~kKnownFlags));
+  if ((desc->flags & LBM_PLAN_ONE_PASS) && (desc->flags & LBM_PLAN_TWO_PASS))
+    return fail(LBM_ERR_INVALID, "plan flags ask for one pass and for two");
   lbm_plan* p = new lbm_plan();
   p->Q = desc->lattice;
   p->D = desc->lattice == LBM_D3Q19 ? 3 : 2;

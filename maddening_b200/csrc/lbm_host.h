@@ -157,13 +157,32 @@ int launch_tiled_pipe(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s)
 template <int Q, class S>
 int launch_tiled_words(const lbm_plan* p, const lbm::StepArgs& a, cudaStream_t s);
 
-// How the one-pass step can take the call: not at all (FP64, a plan that asked
-// for two passes, padded rows, f_out overlapping f_in, which other blocks still
-// read), by bulk copies (rows of a multiple of 4 cells and 16-byte aligned
-// reference-layout buffers), else for D2Q9 by word copies: 1952 x 3047 FP32 122 us
-// against 166 for two passes, 999^2 BF16 35 / 50.  A D3Q19 plane is 250 warp-wide
-// word copies and lost: 255^3 1.66 ms with one producer warp, 1.02 with four,
-// 0.85 in two passes.  status: where its status word goes.
+// Where a D2Q9 lattice takes the one-pass step: it must fill the tiles (rows of
+// kTiledRow9 cells) and be long enough for the ring's latency to hide.  Short or
+// just-over-a-tile rows leave the lanes idle and small lattices are a few planes
+// per block, one after the other, while the two passes then run from the L2.
+// One pass / two passes, us a call (FP32, chained calls in a recorded graph):
+// bulk copies 4096 x 256 34 / 25, 4096 x 128 120 / 108 (8e6 cells: 199 / 208),
+// 1024^2 25 / 26, 1000 x 1048 23 / 25, 1000 x 2097 40 / 56, 512 x 2048 28 / 25,
+// 512 x 4096 48 / 56, 300 x 6990 52 / 57, 256^2 10 / 5; word copies 3 x 21845 73 /
+// 5, 3 x 349525 1045 / 26, 100 x 10485 38 / 25, 301 x 13934 118 / 109, 999 x 1049
+// 27 / 26, 999 x 1574 38 / 43, 1023 x 1537 42 / 43, 1023 x 2050 53 / 57.  Queued
+// calls of the smaller ones cost the same 23 us to issue either way.
+constexpr uint32_t kTiledRow9 = 252;
+inline bool tiled_pays9(const lbm::Geo& g, bool words) {
+  const uint64_t n2 = g.n2, held = (n2 + kTiledRow9 - 1) / kTiledRow9 * kTiledRow9;
+  const uint64_t used = uint64_t(g.ncell) * n2;  // cells x share of the tiles' lanes x held
+  return words ? 3 * n2 >= 2 * held && used >= (uint64_t(5) << 18) * held
+               : 9 * n2 >= 5 * held && used >= (uint64_t(1) << 20) * held;
+}
+
+// How the one-pass step takes the call: not at all (FP64, a plan that asked for
+// two passes, padded rows, f_out overlapping f_in, which other blocks still read,
+// a D2Q9 lattice on which two passes are faster unless the plan asked for one),
+// by bulk copies (rows of a multiple of 4 cells and 16-byte aligned
+// reference-layout buffers), else for D2Q9 by word copies.  A D3Q19 plane is 250
+// warp-wide word copies and lost: 255^3 1.66 ms with one producer warp, 1.02 with
+// four, 0.85 in two passes.  status: where its status word goes.
 enum TiledForm { kTiledNone, kTiledWords, kTiledBulk };
 template <class S>
 TiledForm tiled_form(const lbm_plan* p, const lbm::StepArgs& a, const void* status, bool aos_out) {
@@ -180,6 +199,9 @@ TiledForm tiled_form(const lbm_plan* p, const lbm::StepArgs& a, const void* stat
       if (fo % 4 != 0 || (fo < fi + bytes && fi < fo + bytes)) return kTiledNone;
     }
     const bool aligned = p->g.n2 % 4 == 0 && fi % 16 == 0 && (!aos_out || fo % 16 == 0);
+    if (p->Q == 9 && !(p->flags & (LBM_PLAN_ONE_PASS | LBM_PLAN_TEST_WAIT_TIMEOUT)) &&
+        !tiled_pays9(p->g, !aligned))
+      return kTiledNone;
     return aligned ? kTiledBulk : (p->Q == 9 ? kTiledWords : kTiledNone);
   }
 }

@@ -9,9 +9,13 @@
 
 namespace {
 
+static_assert(lbm::Sweep<9>::TZ == kTiledRow9, "the dispatch rule counts tiles of this length");
+
 // Sweep geometry and work items for a persistent grid of `grid` blocks: the
 // number of chunks along the sweep axis minimises the planes of the busiest
-// block, ceil(items / grid) x (planes per chunk + 2 halo planes).
+// block, ceil(items / grid) x (planes per chunk + 2 halo planes).  Every chunk
+// length is looked at once, with the smallest number of chunks that gives it (128
+// instead of 4096 evaluations for 4096 planes, which took 33 us of host time).
 template <int Q>
 lbm::TileGeo tile_geo(const lbm_plan* p, uint32_t grid) {
   using T = lbm::TileShape<Q>;
@@ -27,8 +31,9 @@ lbm::TileGeo tile_geo(const lbm_plan* p, uint32_t grid) {
   uint64_t best = ~uint64_t(0);
   uint32_t best_chunk = t.NS;
   const uint32_t kmax = std::min<uint32_t>(t.NS, 4096);
-  for (uint32_t k = 1; k <= kmax; ++k) {
+  for (uint32_t k = 1, next; k <= kmax; k = next) {
     const uint32_t chunk = (t.NS + k - 1) / k;
+    next = chunk > 1 ? (t.NS - 1) / (chunk - 1) + 1 : kmax + 1;
     const uint64_t nch = (t.NS + chunk - 1) / chunk;
     const uint64_t items = nch * t.ncol;
     const uint64_t cost = ((items + grid - 1) / grid) * (chunk + 2);

@@ -26,9 +26,11 @@ Additions beyond the reference (documented extensions):
   lattice is large; else one), ``1`` or ``2`` (FP32 with faces too).  Every form
   gives bit-identical results.
 * ``one_pass`` -- ``update`` (and the first step of ``run``) reads the
-  reference-layout ``f`` once in a tiled kernel (``None`` or ``True``, the
-  default; FP32, FP16 and BF16 storage; D3Q19: last extent a multiple of 4) or runs
-  as two passes (``False``); the results are bit-identical.
+  reference-layout ``f`` once in a tiled kernel (``True``; FP32, FP16 and BF16
+  storage; D3Q19: last extent a multiple of 4) or runs as two passes (``False``).
+  ``None``, the default, takes one pass except on D2Q9 lattices that are small or
+  whose rows fill few of the kernel's tiles, where two passes are faster.  The
+  results are bit-identical.
 """
 
 from __future__ import annotations
@@ -156,6 +158,8 @@ class LBMNode(SimulationNode):
             flags |= _lib.PLAN_PAIRED_CELLS
         if one_pass is False:
             flags |= _lib.PLAN_TWO_PASS
+        elif one_pass:
+            flags |= _lib.PLAN_ONE_PASS
         self._plan = _lib.Plan(lat.Q, self._grid_shape, tau, storage, flags)
 
     # -- properties (lbm.py:690-703) ---------------------------------------
