@@ -88,11 +88,14 @@ typedef struct {
                                    (FP16/BF16 storage otherwise takes the
                                    four-cell step on rows of a multiple of 256
                                    cells for D3Q19 / 128 for D2Q9, else the
-                                   paired two-cell step; FP32 storage the paired
-                                   step on even contiguous extents, without
-                                   faces or on large lattices) */
+                                   paired two-cell step, with odd extents only
+                                   where the lattice is large enough for it to be
+                                   faster; FP32 storage the paired step on even
+                                   contiguous extents, without faces or on large
+                                   lattices) */
 #define LBM_PLAN_PAIRED_CELLS 4u /* the paired two-cell step for FP32 storage on
-                                   every even contiguous extent */
+                                   every even contiguous extent, and for 16-bit
+                                   storage on every odd one */
 #define LBM_PLAN_TWO_PASS 8u /* lbm_update and the first step of lbm_rollout run
                                 as two passes (collide into the workspace, then
                                 the pull step) instead of the one-pass tiled

@@ -25,9 +25,20 @@ struct lbm_plan {
   lbm::Geo gpad{};               // the geometry with state rows of n2 + 1 cells
   bool gpad_ok = false;          // ... indexes below 2^32
 
-  // 16-bit states with odd rows are kept padded inside a rollout.
-  bool odd_rows_padded() const {
-    return elem == 2 && g.n2 % 2 == 1 && gpad_ok && !(flags & LBM_PLAN_SINGLE_CELLS);
+  // 16-bit states with odd rows are kept padded inside a rollout where two cells per
+  // thread gain more than the padding cell costs (faces: whether the call has face
+  // conditions; without them the plan's workspace is sized for it), and wherever the
+  // plan asks for pairs.  us of 20 steps, padded pairs / one cell per thread, FP16:
+  // without faces 24^3 45.8 / 44.8, 33^3 50.5 / 54.9, 48 x 48 x 49 73 / 91, 200 x 200 x
+  // 199 2538 / 3212, 999^2 178 / 229, 200 x 200 x 5 89 / 108, 512 x 512 x 5 525 / 526,
+  // 1024 x 1024 x 3 1337 / 1233, 512 x 512 x 1 153 / 128; with faces, whose own code
+  // runs for both cells of a pair, 33^3 138 / 101, 64 x 64 x 63 192 / 180, 80 x 80 x 81
+  // 269 / 281, 700 x 701 156 / 167, 300 x 300 x 15 627 / 616, 300 x 300 x 31 1138 / 1191.
+  bool odd_rows_padded(bool faces) const {
+    if (elem != 2 || g.n2 % 2 == 0 || !gpad_ok || (flags & LBM_PLAN_SINGLE_CELLS)) return false;
+    if (flags & LBM_PLAN_PAIRED_CELLS) return true;
+    if (faces) return g.n2 > 16 && g.ncell >= (3u << 17);
+    return g.n2 >= 3 && g.ncell >= (1u << 15) && (g.n2 >= 7 || g.ncell < (1u << 20));
   }
 };
 
@@ -47,7 +58,7 @@ inline size_t padded_state_bytes(const lbm_plan* p) {
 }
 // Workspace of a rollout of more than one step: two state copies, a status word.
 inline size_t rollout_bytes(const lbm_plan* p) {
-  const size_t sb = p->odd_rows_padded() ? padded_state_bytes(p) : state_bytes(p);
+  const size_t sb = p->odd_rows_padded(false) ? padded_state_bytes(p) : state_bytes(p);
   return 2 * align256(sb) + 256;
 }
 

@@ -249,12 +249,10 @@ int run_steps(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* f_
               int64_t n, char* ws, size_t ws_bytes) {
   size_t sb = align256(state_bytes(p));
   if (n > 1 && ws_bytes >= rollout_bytes(p) && reinterpret_cast<uintptr_t>(ws) % 4 == 0 &&
-      p->odd_rows_padded()) {
+      p->odd_rows_padded(a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone)) {
     // 16-bit state with odd rows: a padding cell per row lets the steps run two
-    // cells per thread (BF16 149 x 111 x 93: 30.3 us a step against 34.0 with one
-    // cell per thread; FP16 201^3 140.9 / 168.2; 999^2 8.7 / 12.6).  A workspace
-    // without room for the padding, or off the 4-byte boundaries that a pair's
-    // accesses need, keeps one cell.
+    // cells per thread.  A workspace without room for the padding, or off the 4-byte
+    // boundaries that a pair's accesses need, keeps one cell.
     a.g = p->gpad;
     sb = align256(padded_state_bytes(p));
   }

@@ -21,10 +21,11 @@ Additions beyond the reference (documented extensions):
   ``"f32"`` (default), ``"f16"``/``"bf16"`` (normalised offsets, FP32
   arithmetic) or ``"f64"`` (FP64 throughout; state arrays are float64).
 * ``cells_per_thread`` -- kernel form of the steps inside ``run``: ``None``
-  (default: two neighbouring cells per thread, or four, for FP16/BF16 storage;
-  for FP32 two when the contiguous extent is even and there are no faces or the
-  lattice is large; else one), ``1`` or ``2`` (FP32 with faces too).  Every form
-  gives bit-identical results.
+  (default: two neighbouring cells per thread, or four, for FP16/BF16 storage,
+  with an odd contiguous extent on large lattices only; for FP32 two when the
+  contiguous extent is even and there are no faces or the lattice is large; else
+  one), ``1`` or ``2`` (wherever a two-cell form exists).  Every form gives
+  bit-identical results.
 * ``one_pass`` -- ``update`` (and the first step of ``run``) reads the
   reference-layout ``f`` once in a tiled kernel (``True``; FP32, FP16 and BF16
   storage; D3Q19: last extent a multiple of 4) or runs as two passes (``False``).

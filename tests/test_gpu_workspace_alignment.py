@@ -12,10 +12,12 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("shape", [(5, 4, 3), (6, 7, 129), (4, 6, 66), (9, 1), (8, 257), (6, 130)])
 @pytest.mark.parametrize("storage", ["f16", "bf16"])
-def test_workspace_on_a_two_byte_boundary(shape, storage):
+@pytest.mark.parametrize("cells", [None, 2])
+def test_workspace_on_a_two_byte_boundary(shape, storage, cells):
     from maddening_b200 import LBMNode, _lib
     rng = np.random.default_rng(5)
     node = LBMNode("w", 1.0, grid_shape=shape, viscosity=0.05, storage=storage,
+                   cells_per_thread=cells,
                    lattice="D3Q19" if len(shape) == 3 else "D2Q9",
                    wall_mask=rng.random(shape) < 0.15)
     st, dev = node.initial_state(), torch.device("cuda")
