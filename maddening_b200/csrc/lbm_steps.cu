@@ -373,13 +373,12 @@ int run_history(const lbm_plan* p, cudaStream_t s, lbm::StepArgs a, const void* 
 template <int Q, class S>
 int state_op(StateOp op, const lbm::StepArgs& a, cudaStream_t s) {
   if (op == kFromF) return launch_prepare<Q, S>(a, s);
-  if (op == kStep) {
-    // one cell per thread, any storage; an ordinary launch: the caller orders these
-    // steps against exchanges on other streams
-    launch_step_mode<Q, S, lbm::kOutState, false>(a, s);
-    return cuda_check(cudaGetLastError(), "k_step launch");
-  }
-  return launch_step<Q, S>(a, true, s);
+  // One cell per thread, any storage.  Ordinary launches: the caller orders these
+  // steps against exchanges on other streams, and across such a wait a launch
+  // ahead of the step before has nothing to hide.
+  if (op == kStep) launch_step_mode<Q, S, lbm::kOutState, false>(a, s);
+  else launch_step_mode<Q, S, lbm::kOutAoS, false>(a, s);
+  return cuda_check(cudaGetLastError(), "k_step launch");
 }
 
 #define LBM_UNIT(Q, S)                                                                        \
