@@ -31,12 +31,14 @@ void launch_step_mode(const lbm::StepArgs& a, cudaStream_t s) {
 // Paired-cell state step (lbm_pair.cuh): the default for 16-bit storage; for FP32
 // without faces, or on lattices large enough that the faces' own code is few
 // warps' work; always with LBM_PLAN_PAIRED_CELLS, never with
-// LBM_PLAN_SINGLE_CELLS.  FP32 us a step with two cells / one cell per thread,
-// force without faces: 48^3 2.97 / 4.27, 96^3 19.9 / 22.7, 256^3 379 / 392, 1024^2
-// 8.4 / 12.4, 2048^2 48.4 / 50.9; with faces: 64^3 8.1 / 7.6, 96^3 23.3 / 23.9,
-// 128^3 53.6 / 53.1, 160^3 100.1 / 100.8, 256^3 383 / 393; 512^2 4.6 / 4.5, 1024^2
-// 9.9 / 12.6.  Rows of even length; state planes and the wall mask aligned for
-// the pair width.
+// LBM_PLAN_SINGLE_CELLS.  FP32 us a step of a 20-step rollout with two cells / one
+// cell per thread: without faces 64^3 5.7 / 6.5, 96^3 21.3 / 23.3, 256^3 396 / 424,
+// 512^2 3.8 / 4.5, 1024^2 9.5 / 11.9.  With faces, D3Q19: 64^3 9.5 / 8.5, 80^3 14.0 /
+// 13.3, 96^3 24.6 / 25.1, 112^3 40.1 / 39.2, 128^3 57.1 / 56.9, 144^3 79.1 / 78.5, 160^3
+// 105 / 107, 176^3 140 / 143, 200^3 197 / 204, 256^3 404 / 428: 2 % either way between
+// 96^3 and 160^3, a gain beyond.  D2Q9: 362^2 5.1 / 4.4, 512^2 5.6 / 5.5, 600^2 6.4 /
+// 6.4, 700^2 7.3 / 7.8, 800^2 8.4 / 9.4, 960^2 10.7 / 12.3, 1024^2 11.4 / 13.8.
+// Rows of even length; state planes and the wall mask aligned for the pair width.
 template <int Q, class S>
 bool pair_ok(const lbm_plan* p, const lbm::StepArgs& a) {
   if constexpr (sizeof(S) == 8) {
@@ -46,7 +48,7 @@ bool pair_ok(const lbm_plan* p, const lbm::StepArgs& a) {
     if (sizeof(S) == 4 && !(p->flags & LBM_PLAN_PAIRED_CELLS)) {
       const bool faces =
           a.face[0].kind != lbm::kFaceNone || a.face[1].kind != lbm::kFaceNone;
-      if (faces && p->g.ncell < (Q == 9 ? 1u << 20 : 1u << 22)) return false;
+      if (faces && p->g.ncell < (Q == 9 ? 1u << 19 : 1u << 22)) return false;
     }
     const uintptr_t al = 2 * sizeof(S);
     return p->g.n2 % 2 == 0 && reinterpret_cast<uintptr_t>(a.pin) % al == 0 &&
@@ -85,9 +87,9 @@ void launch_quad_w(const lbm::StepArgs& a, cudaStream_t s) {
 
 // The four-cell form (16-bit storage): rows of a multiple of 128 cells,
 // unpadded state rows, 8-byte aligned planes and a 4-byte aligned wall mask.
-// D3Q19 also takes it (a B200 sweep at 256^3: 79.2k MLUPS FP16 against 71.7k
-// for pairs, at 20 resident warps and 96 registers) on rows of a multiple of
-// 256 cells: with one-warp blocks (rows of 128) it keeps 15 warps resident and
+// D3Q19 also takes it (a B200 sweep at 256^3 with one-wide arithmetic: 79.2k MLUPS
+// FP16 against 71.7k for pairs; register budgets at quad_min_warps) on rows of a
+// multiple of 256 cells: with one-warp blocks (rows of 128) it keeps 15 warps resident and
 // loses to pairs.
 #ifndef LBM_QUAD_Q19
 #define LBM_QUAD_Q19 1
