@@ -300,9 +300,10 @@ int lbm_pipe_rollout(const lbm_plan* plan, lbm_stream_t stream, const void* f_in
  * a checkpoint of the populations every `checkpoint_every` steps (<= 0: the
  * ceiling of sqrt(n_steps)) in the workspace, and the backward recomputes each
  * segment storing only (rho, u) per step, then runs the hand-written adjoint
- * step.  Where (rho, u) of every step take no more room than that (short
- * rollouts, checkpoint_every >= n_steps), the forward keeps those instead and
- * nothing is recomputed.  The workspace must stay untouched between the two
+ * step.  Where (rho, u) of every step take no more room than that (at the default
+ * interval up to 40 steps and 43 to 45 with D3Q19, up to 23 with D2Q9; any count
+ * with checkpoint_every >= n_steps, which asks for it), the forward keeps those
+ * instead and nothing is recomputed.  The workspace must stay untouched between the two
  * calls. */
 int lbm_adjoint_workspace_bytes(const lbm_plan* plan, int64_t n_steps, int64_t checkpoint_every,
                                 size_t* bytes);

@@ -152,7 +152,7 @@ struct StepArgs {
   void* vel;
   void* prs;
   uint32_t mflags;
-  int* status;  // device word; bit 0 set when a bounded wait gave up (staged path)
+  int* status;  // device word; bit 0 set when a bounded wait gave up (one-pass kernel)
   // Face planes sit this many cells inside the lattice: 0, or 1 for a
   // halo-padded block (the faces act on the interior).
   uint32_t face_inset;

@@ -23,8 +23,8 @@
 //                 place: every warp store is one aligned 128-byte run.
 // The first step collides the reference f (read through shared memory in
 // its (grid, 19) layout); the last pass pulls the state into the reference
-// f_bc and the outputs.  Every sum runs in the order of the push form this
-// replaced (f_str before the wall swap), so the outputs are bit-identical.
+// f_bc and the outputs.  Every sum runs over f_str, before the wall swap, as the
+// reference's does.
 // Traffic per cell and step: 19 loads + 1 psi store, then 19 loads + 19
 // stores + the psi loads (mostly cache hits).
 #pragma once

@@ -38,9 +38,10 @@
 // Requirements (checked on the host): 32-bit IO (FP32, FP16 or BF16 storage),
 // f_in and f_out not overlapping, no halo-padded block; the bulk copies want an
 // a2 extent that is a multiple of 4 and f_in (and f_out for kOutAoS) 16-byte
-// aligned, the word-copy form (D2Q9 update) neither.  Every wait is bounded in time and also ends when another warp
-// has given up; then the block sets bit 0 of *status, waits (bounded) for its
-// own copies in flight, fills its output cells with NaN and returns.
+// aligned, the word-copy form (D2Q9 update) neither.  Every wait is bounded in
+// time and also ends when another warp has given up; then the block sets bit 0 of
+// *status, waits (bounded) for its own copies in flight, fills its output cells
+// with NaN and returns.
 #pragma once
 
 #include <type_traits>
@@ -409,9 +410,9 @@ __device__ __forceinline__ float cell_of(float v) { return v; }
 template <int J>
 __device__ __forceinline__ float cell_of(F2 v) { return J == 0 ? v.v.x : v.v.y; }
 
-// A wall byte, loaded where the source places it: the output warps fetch the
-// next plane's byte one plane ahead, and a volatile load is neither moved
-// towards its use nor repeated there by the compiler.
+// A wall byte, loaded where the source places it: the collide warps fetch the
+// bytes of their cells ahead of the wait for the plane, and a volatile load is
+// neither moved towards its use nor repeated there by the compiler.
 __device__ __forceinline__ uint8_t ld_wall(const uint8_t* p) {
   uint16_t v;
   asm volatile("ld.global.nc.u8 %0, [%1];" : "=h"(v) : "l"(p));

@@ -536,10 +536,11 @@ class LBMNode(SimulationNode):
 
         Populations are checkpointed every ``checkpoint_every`` steps (0: the
         ceiling of sqrt(n_steps)) and the backward recomputes each segment; where
-        the density and velocity of every step take no more memory than that (short
-        rollouts, or ``checkpoint_every >= n_steps``) they are kept instead and
-        nothing is recomputed.  Walls
-        and body forces only (no face conditions); FP32 or FP64 storage.
+        the density and velocity of every step take no more memory than that (by
+        default up to 40 steps and 43 to 45 with D3Q19, up to 23 with D2Q9) they are
+        kept instead and nothing is recomputed; ``checkpoint_every >= n_steps`` asks
+        for that at any length (16 bytes per cell and step in FP32).  Walls and body forces
+        only (no face conditions); FP32 or FP64 storage.
         """
         if int(n_steps) < 1:
             raise ValueError("n_steps must be >= 1")
